@@ -50,9 +50,9 @@ int unit_slots(const dc_ctx* c) { return c->opt.unit_slots; }
 dc_status ensure_recolor_scratch(dc_ctx* ctx) {
   if (ctx->rc_pool_cap == ctx->pool_cap) return DC_OK;
   const long long n = std::max(ctx->n, 1);
-  // the loop cuts units down to an eighth of unit_slots (at least 128) when
-  // a frontier is small
-  const long long CH = std::max<long long>(128, (unit_slots(ctx) / 8) & ~127ll);
+  // units are cut down to an eighth of unit_slots (at least 128) when a
+  // seeding phase is small, and to kLoopUnit in the loop
+  const long long CH = std::min<long long>(kLoopUnit, std::max<long long>(128, (unit_slots(ctx) / 8) & ~127ll));
   const long long capU = n + ctx->pool_cap / CH + 64;
   // mask words: a multi-unit row (length L > its unit size) takes at most
   // L/32 + 7 words in the mex modes and 132 words for saturation sizes
@@ -95,6 +95,7 @@ dc_status ensure_recolor_scratch(dc_ctx* ctx) {
       if ((s = dalloc(ctx, &h.xv, h.cap_exc, "change lists")) != DC_OK) return s;
       if ((s = dalloc(ctx, &h.alist, h.cap_a, "append queue")) != DC_OK) return s;
       if ((s = dalloc(ctx, &h.hist, h.cap_hist * kHriBins, "heavy-row colour counts")) != DC_OK) return s;
+      if ((s = dalloc(ctx, &h.hstart, h.cap_hist * kHriBins, "heavy-row colour starts")) != DC_OK) return s;
     } else {
       if ((s = dalloc(ctx, &h.ids, h.cap_pairs, "split neighbours")) != DC_OK) return s;
     }
@@ -105,6 +106,11 @@ dc_status ensure_recolor_scratch(dc_ctx* ctx) {
     if ((s = dalloc(ctx, &ctx->bmC, words, "bitmap")) != DC_OK) return s;
     if ((s = dalloc(ctx, &ctx->ncolor, n, "ncolor")) != DC_OK) return s;
     if ((s = dalloc(ctx, &ctx->sat, n, "sat")) != DC_OK) return s;
+    // the loop rebuilds the member list before its dead entries pass half of
+    // the live ones plus kMemSlack
+    ctx->mem_cap = n + n / 2 + 2 * kMemSlack;
+    if ((s = dalloc(ctx, &ctx->mem, ctx->mem_cap, "frontier members")) != DC_OK) return s;
+    if ((s = dalloc(ctx, &ctx->mout, n, "frontier changes")) != DC_OK) return s;
     if (ctx->opt.variant == DC_HB && (s = dalloc(ctx, &ctx->cp, n, "packed words")) != DC_OK) return s;
     if (ctx->opt.heavy_min_live > 0) {
       HriBufs& h = ctx->hri;
@@ -249,6 +255,9 @@ RecolorParams recolor_params(dc_ctx* ctx, const dc_change* ch, long long k) {
   p.bmC = ctx->bmC;
   p.ncolor = ctx->ncolor;
   p.sat = ctx->sat;
+  p.mem = ctx->mem;
+  p.mem_cap = ctx->mem_cap;
+  p.mout = ctx->mout;
   p.cp = ctx->cp;
   p.hri = ctx->hri;
   p.lflag = ctx->lflag;
@@ -689,6 +698,8 @@ void dc_destroy(dc_ctx* ctx) {
   dfree(ctx, &ctx->bmC);
   dfree(ctx, &ctx->ncolor);
   dfree(ctx, &ctx->sat);
+  dfree(ctx, &ctx->mem);
+  dfree(ctx, &ctx->mout);
   dfree(ctx, &ctx->cp);
   dfree(ctx, &ctx->hri.hid);
   dfree(ctx, &ctx->hri.bmF);
@@ -701,6 +712,7 @@ void dc_destroy(dc_ctx* ctx) {
   dfree(ctx, &ctx->hri.xv);
   dfree(ctx, &ctx->hri.alist);
   dfree(ctx, &ctx->hri.hist);
+  dfree(ctx, &ctx->hri.hstart);
   dfree(ctx, &ctx->hri.hsplit);
   dfree(ctx, &ctx->hri.bcnt);
   dfree(ctx, &ctx->d_ranges);

@@ -60,6 +60,9 @@ struct dc_ctx {
   unsigned* bmC = nullptr;
   int* ncolor = nullptr;
   int* sat = nullptr;
+  int* mem = nullptr;      // frontier member list of the recolour loop
+  long long mem_cap = 0;
+  int* mout = nullptr;     // members the loop's commit touches
   unsigned long long* cp = nullptr;  // HB: packed (degree property, colour) per vertex
   HriBufs hri{};                     // HI: heavy-row index (min_live 0: off)
 

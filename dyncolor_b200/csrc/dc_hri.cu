@@ -191,6 +191,11 @@ __global__ void __launch_bounds__(kHriThreads) hri_fill_kernel(GraphDev g, HriBu
       __syncthreads();
       hist[b0] = start;  // becomes the bin's write cursor
       hist[b1] = start + c0;
+      if (i < h.cap_hist) {
+        // a pushing row's bounds in its copy
+        h.hstart[i * kHriBins + b0] = start;
+        h.hstart[i * kHriBins + b1] = start + c0;
+      }
     }
     __syncthreads();
     for (int s = threadIdx.x; s < L; s += kHriThreads) {

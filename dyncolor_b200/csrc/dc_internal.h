@@ -24,23 +24,47 @@ constexpr int kMaskWords = 128;     // colour window per warp: 4096 colours
 constexpr int kMaskBits = kMaskWords * 32;
 constexpr int kStructChunk = 1024;  // slots per unit in the structural row scans
 constexpr int kTomb = -1;           // tombstoned adjacency slot
-// During the recolour loop, bit 30 of color[v] marks v for the next
-// frontier; colours are below 2^30.  The commit's store clears it.
+// During the recolour loop the colour word of v (color[v] for HI, the low
+// half of cp[v] for HB) carries two flags above the colour, which is below
+// 2^30: bit 30 marks v as new in the next frontier (the commit clears it),
+// bit 31 says that v is in the current frontier.
 constexpr unsigned kMarkBit = 1u << 30;
+constexpr unsigned kInF = 1u << 31;
 constexpr int kColorMask = (1 << 30) - 1;
-constexpr int kNumQueues = 6;       // logical queue counter slots
+constexpr int kNumQueues = 8;       // logical queue counter slots
+constexpr long long kMemSlack = 4096;     // member-list entries the loop may add beyond half the live ones before a rebuild
 constexpr int kUnitSlotsDefault = 4096;  // adjacency slots per warp work unit
+constexpr int kLoopUnit = 512;           // slots per work unit of the recolour loop's rows, at most
 constexpr long long kLoadPiece = 1ll << 27;  // edge pairs per structural launch of a graph load
 constexpr int kBarrierTimeoutMsDefault = 20000;  // grid-barrier wait limit unless the options set one
 
-// Logical queue counter slots.
-enum { Q_LOOP0 = 0, Q_LOOP1 = 1, Q_LOOP2 = 2, Q_S1 = 3, Q_S2E = 4, Q_S2T = 5 };
+// Logical queue counter slots.  Loop: Q_PUSH rows that push their marks in
+// this iteration, Q_SCAN long rows whose members look for a new witness,
+// Q_EVAL + iteration % 3 rows whose mex is computed.  Seeding: Q_S*.
+enum { Q_PUSH = 0, Q_SCAN = 1, Q_EVAL = 2, Q_S1 = 5, Q_S2E = 6, Q_S2T = 7 };
 
 struct QCount {
-  unsigned long long countA;  // class A items
-  unsigned long long countU;  // work units (class B/C)
-  unsigned long long masks;   // multi-unit mask words handed out
-  unsigned long long pad;
+  unsigned countA;  // class A items
+  unsigned countU;  // work units (class B/C)
+  unsigned masks;   // multi-unit mask words handed out
+  unsigned pad;
+};
+
+// Counters of the recolour and initial-colouring launches.
+struct LoopState {
+  QCount q[kNumQueues];
+  // frontier member list and per-iteration counters (rings of three by
+  // iteration, so a counter is cleared two iterations after its last reader)
+  unsigned m_tail;       // entries in the member list, this iteration's entrants included
+  unsigned m_build;      // entries written while the list is rebuilt
+  unsigned m_len[3];     // entries at the start of the iteration
+  unsigned m_live[3];    // members at the start of the iteration
+  unsigned ev_rows[3];   // rows of the EVAL queue
+  unsigned m_out[3];     // members that leave
+  unsigned a_count;      // (vertex, chunk) items waiting for the append phase
+  unsigned m_rebuild[3]; // 1: rebuild the member list before the iteration
+  int chg[3];            // "a colour changed" flags
+  unsigned pad;
 };
 
 // Lives in device memory.  Fields up to `pool_used_start` persist across
@@ -55,8 +79,7 @@ struct DevState {
   // ---- cleared before every kernel launch (bar_arrived .. wctr) ----
   unsigned bar_arrived;
   unsigned bar_abort;
-  int chg[2];                      // HB loop: "a colour changed" flags, ring by iteration
-  unsigned long long wctr[3];      // work-grab counters (ring by phase)
+  unsigned wctr[4];                // work-grab counters (ring of three by phase)
   // ---- cleared before every batch (bar_arrived .. end) ----
   unsigned status;
   unsigned pre_status;             // status of the structural launch, copied before the recolour launch
@@ -68,7 +91,7 @@ struct DevState {
   unsigned long long nunits;       // row-scan units
   unsigned long long nrel;         // relocation copy units
   // recolour kernel
-  QCount q[kNumQueues];
+  LoopState ls;
   // statistics
   unsigned long long iterations;
   unsigned long long seed_targets;
@@ -83,10 +106,8 @@ struct DevState {
   unsigned long long phase_ns[6];     // recolour launch: seeding, find-eligible, mex, commit, 2 spare
   // heavy-row index
   unsigned long long hcount;          // rows found with at least min_live live slots
-  unsigned long long a_count;         // (vertex, chunk) items waiting for the append phase
   unsigned hri_off;                   // 1: the index is incomplete for this batch; full scans only
   unsigned pad1;
-  long long read_delta;               // adjacency/index entries read minus entries scanned
 };
 
 struct GraphDev {
@@ -172,6 +193,7 @@ struct HriBufs {
   int2* alist;                // cap_a: (vertex, chunk) of first changes, for the append phase
   int* hist;                  // cap_hist * kHriBins: row i's count of neighbours per launch-start colour
                               // that have not changed colour since (the append phase takes them off)
+  int* hstart;                // cap_hist * kHriBins: entries of row i's copy above each colour
   int* hsplit;                // HB, cap_rows: row i's copy (in ids) holds its prior neighbours first,
                               // hsplit[i] of them, then the rest
   unsigned long long* bcnt;   // 64: rows per length class, then the classes' cursors (build scratch)
@@ -198,7 +220,10 @@ struct RecolorParams {
   unsigned* bmB;
   unsigned* bmC;
   int* ncolor;           // n
-  int* sat;              // n
+  int* sat;              // n: saturation sizes (seeding), then each member's witness (loop)
+  int* mem;              // mem_cap: frontier member list (-1: left)
+  long long mem_cap;
+  int* mout;             // n: the iteration's members that leave
   unsigned long long* cp;  // HB: n packed (degree property, colour) words
   HriBufs hri;             // HI: heavy-row index (hri.min_live == 0: off)
   unsigned char* lflag;  // k

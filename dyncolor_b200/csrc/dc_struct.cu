@@ -313,8 +313,8 @@ __global__ void __launch_bounds__(kThreads) struct_kernel(StructParams p) {
   {
     const long long NU = min((long long)ld_cg(&st->nunits), p.cap_units);
     while (true) {
-      unsigned long long ui = 0;
-      if (lane == 0) ui = atomicAdd(&st->wctr[0], 1ull);
+      unsigned ui = 0;
+      if (lane == 0) ui = atomicAdd(&st->wctr[0], 1u);
       ui = __shfl_sync(0xffffffffu, ui, 0);
       if ((long long)ui >= NU) break;
       const int2 u = p.units[ui];
@@ -465,8 +465,8 @@ __global__ void __launch_bounds__(kThreads) struct_kernel(StructParams p) {
   {
     const long long NR = min((long long)ld_cg(&st->nrel), p.cap_rel);
     while (true) {
-      unsigned long long ui = 0;
-      if (lane == 0) ui = atomicAdd(&st->wctr[1], 1ull);
+      unsigned ui = 0;
+      if (lane == 0) ui = atomicAdd(&st->wctr[1], 1u);
       ui = __shfl_sync(0xffffffffu, ui, 0);
       if ((long long)ui >= NR) break;
       const int2 u = p.relunits[ui];

@@ -93,7 +93,7 @@ typedef struct {
   int64_t iterations;     /* executions of the recolour loop body */
   int64_t seed_targets;   /* distinct vertices recomputed by the seeding steps */
   int64_t frontier_total; /* sum over iterations of the recolour frontier size */
-  int64_t slots_scanned;  /* live adjacency entries read by seeding + loop */
+  int64_t slots_scanned;  /* live adjacency entries the rules of seeding + loop cover */
   int64_t edges_inserted; /* net structural insertions (new edges) */
   int64_t edges_deleted;  /* net structural deletions (edges removed) */
   int64_t rows_relocated; /* adjacency rows moved to new capacity */
@@ -104,8 +104,10 @@ typedef struct {
   double recolor_ms;      /* of which the seeding + recolour launch */
   double phase_ms[6];     /* recolour launch split: seeding, find-eligible, mex, commit,
                              2 reserved */
-  int64_t slots_read;     /* adjacency entries the kernels actually read (the loop
-                             reads each frontier row once per iteration) */
+  int64_t slots_read;     /* of slots_scanned, the entries that no index stood in for: rows the
+                             heavy-row index covers count by the entries read through it, other
+                             rows in full (the loop skips most of those too: it reads a row only
+                             where a mark or a colour can have changed) */
   int64_t pairs;          /* frontier-internal edges the fused loop deferred */
 } dc_stats;
 
