@@ -274,12 +274,10 @@ RecolorParams recolor_params(dc_ctx* ctx, const dc_change* ch, long long k) {
   return p;
 }
 
-// Clears the per-launch part of DevState and snapshots the pool counter.
+// Clears the per-batch part of DevState.
 dc_status reset_state(dc_ctx* ctx) {
-  const size_t off = offsetof(DevState, bar_arrived);
+  const size_t off = offsetof(DevState, ctl);
   DC_CK(cudaMemsetAsync(reinterpret_cast<char*>(ctx->st) + off, 0, sizeof(DevState) - off, ctx->stream));
-  DC_CK(cudaMemcpyAsync(&ctx->st->pool_used_start, &ctx->st->pool_used, sizeof(unsigned long long),
-                        cudaMemcpyDeviceToDevice, ctx->stream));
   return DC_OK;
 }
 
@@ -390,7 +388,15 @@ dc_status repack(dc_ctx* ctx, long long new_cap) {
   return DC_OK;
 }
 
-// Runs one batch (or a load) already resident on the device.
+// CTAs of the structural launch.  Its barriers cost more with more CTAs (1.0
+// us each at one per SM, 1.8 at two), its row scans and sort passes run faster:
+// 5k lines 125 us at one per SM and 144 at two, 20k lines 164 and 198, 100k
+// lines 577 and 405; the two lines cross near 31k.
+constexpr long long kOneCtaPerSmLines = 32768;
+int struct_grid(const dc_ctx* ctx, long long k) {
+  return k <= kOneCtaPerSmLines ? std::min(ctx->grid_struct, ctx->sms) : ctx->grid_struct;
+}
+
 // Enqueues one attempt of a batch (or load) on the context's stream, ending
 // with the copy of the device state into pinned host memory.  k_dev, when
 // set, makes the kernels read the line count from device memory, so a
@@ -403,7 +409,8 @@ dc_status enqueue_batch(dc_ctx* ctx, const dc_change* d_ch, const int* la, const
   if ((s = reset_state(ctx)) != DC_OK) return s;
   StructParams sp = struct_params(ctx, d_ch, la, lb, k);
   sp.k_dev = k_dev;
-  DC_CK(launch_struct(sp, ctx->grid_struct, ctx->stream));
+  // (a captured sequence serves every batch that the scratch can hold)
+  DC_CK(launch_struct(sp, struct_grid(ctx, k_dev ? ctx->kcap : k), ctx->stream));
   if (events) DC_CK(cudaEventRecord(ctx->evm, ctx->stream));
   if (recolor) {
     if (ctx->ngraphs > 0) {
@@ -413,12 +420,6 @@ dc_status enqueue_batch(dc_ctx* ctx, const dc_change* d_ch, const int* la, const
       DC_CK(cudaMemsetAsync(ctx->giters, 0, G * sizeof(int), ctx->stream));
       DC_CK(cudaMemsetAsync(ctx->gstate, 0, G * sizeof(int), ctx->stream));
     }
-    DC_CK(cudaMemcpyAsync(&ctx->st->pre_status, &ctx->st->status, sizeof(unsigned),
-                          cudaMemcpyDeviceToDevice, ctx->stream));
-    // fresh grid barrier and work counters for the second cooperative launch
-    const size_t b0 = offsetof(DevState, bar_arrived);
-    const size_t b1 = offsetof(DevState, wctr) + sizeof(((DevState*)nullptr)->wctr);
-    DC_CK(cudaMemsetAsync(reinterpret_cast<char*>(ctx->st) + b0, 0, b1 - b0, ctx->stream));
     RecolorParams rp = recolor_params(ctx, d_ch, k);
     rp.k_dev = k_dev;
     rp.ranges = ctx->index_n > 0 ? ctx->d_ranges : nullptr;
@@ -857,7 +858,7 @@ dc_status dc_colors_init(dc_ctx* ctx, int32_t order) {
     e = cudaMemsetAsync(prio, 0, (size_t)n * 4, ctx->stream);
   if (e == cudaSuccess) {
     // fresh counters, queues and grid barrier for the launch
-    const size_t off = offsetof(DevState, bar_arrived);
+    const size_t off = offsetof(DevState, ctl);
     e = cudaMemsetAsync(reinterpret_cast<char*>(ctx->st) + off, 0, sizeof(DevState) - off, ctx->stream);
   }
   if (e == cudaSuccess) e = cudaMemsetAsync(&ctx->st->cmax, 0, sizeof(int), ctx->stream);

@@ -51,33 +51,25 @@ __device__ __forceinline__ T ld_cg(const T* p) {
 // hanging.  Measured with 296 CTAs whose threads all have a store in flight:
 // 1.71 us per barrier; with a full fence before a plain atomic, and a 64 ns
 // sleep between polls, 2.04 us.
-__device__ __forceinline__ bool barrier_wait(DevState* st, unsigned& target, unsigned long long timeout_ns) {
+__device__ __forceinline__ bool barrier_wait(DevState* st, LaunchCtl* ctl, unsigned& target,
+                                             unsigned long long timeout_ns) {
   target += gridDim.x;
-  asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&st->bar_arrived) : "memory");
+  asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&ctl->bar_arrived) : "memory");
   const unsigned long long t0 = globaltimer_ns();
   unsigned spins = 0;
-  while ((int)(ld_acquire_u32(&st->bar_arrived) - target) < 0) {
+  while ((int)(ld_acquire_u32(&ctl->bar_arrived) - target) < 0) {
     if ((++spins & 15u) == 0) {
-      if (ld_volatile_u32(&st->bar_abort)) return false;
+      if (ld_volatile_u32(&ctl->bar_abort)) return false;
       if ((spins & 255u) == 0 && globaltimer_ns() - t0 > timeout_ns) {
         atomicOr(&st->status, ST_TIMEOUT);
-        atomicExch(&st->bar_abort, 1u);
+        atomicOr(&st->pre_status, ST_TIMEOUT);
+        atomicExch(&ctl->bar_abort, 1u);
         return false;
       }
     }
     __nanosleep(20);
   }
-  return ld_volatile_u32(&st->bar_abort) == 0u;
-}
-
-// The grid barrier; `target` is per-CTA state starting at 0.  All threads
-// call; false once a wait has run out.
-__device__ __forceinline__ bool grid_sync(DevState* st, unsigned& target, unsigned long long timeout_ns) {
-  __shared__ int s_ok;
-  __syncthreads();
-  if (threadIdx.x == 0) s_ok = barrier_wait(st, target, timeout_ns) ? 1 : 0;
-  __syncthreads();
-  return s_ok != 0;
+  return ld_volatile_u32(&ctl->bar_abort) == 0u;
 }
 
 __device__ __forceinline__ int warp_incl_scan(int x) {

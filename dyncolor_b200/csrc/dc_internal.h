@@ -67,22 +67,26 @@ struct LoopState {
   unsigned pad;
 };
 
-// Lives in device memory.  Fields up to `pool_used_start` persist across
-// batches; everything from `bar_arrived` on is cleared before every batch,
-// and bar_arrived .. wctr again before every launch.
+// Grid barrier and work-grab counters of one cooperative launch.
+struct LaunchCtl {
+  unsigned bar_arrived;
+  unsigned bar_abort;
+  unsigned wctr[4];  // ring of three by phase
+  unsigned pad[2];
+};
+
+// Lives in device memory.  Fields up to `ctl` persist across batches; the
+// rest is cleared before every batch (each launch of a batch has its own
+// barrier, so nothing is cleared between them).
 struct DevState {
   int cmax;                        // upper bound of every colour value
   int pad0;
   unsigned long long pool_used;    // adjacency pool slots handed out
   long long batch_k;               // line count, read by kernels of a captured batch graph
-  unsigned long long pool_used_start;
-  // ---- cleared before every kernel launch (bar_arrived .. wctr) ----
-  unsigned bar_arrived;
-  unsigned bar_abort;
-  unsigned wctr[4];                // work-grab counters (ring of three by phase)
-  // ---- cleared before every batch (bar_arrived .. end) ----
+  // ---- cleared before every batch (ctl .. end) ----
+  LaunchCtl ctl[2];                // the structural launch, the recolour launch
   unsigned status;
-  unsigned pre_status;             // status of the structural launch, copied before the recolour launch
+  unsigned pre_status;             // nonzero: the structural launch failed, the batch is not applied
   // structural kernel
   unsigned long long nvalid;       // valid change lines
   unsigned long long nnet;         // netted (row, nbr) entries

@@ -1831,7 +1831,7 @@ __device__ __noinline__ bool sync_grid(DevState* st, unsigned long long timeout_
   Shared& sh = shared();
   __syncthreads();
   if (warp_id() == 0) {
-    if (lane_id() == 0) sh.ok = barrier_wait(st, sh.bar, timeout_ns) ? 1 : 0;
+    if (lane_id() == 0) sh.ok = barrier_wait(st, &st->ctl[1], sh.bar, timeout_ns) ? 1 : 0;
     __syncwarp();
 #pragma unroll
     for (int i = 0; i < kStateWords; i += 32)
@@ -1985,9 +1985,9 @@ __global__ void __launch_bounds__(kThreads, 2) recolor_kernel(const __grid_const
     }
     // Counter the warps take work items from; the next phase's, last used two
     // phases ago, is cleared.
-    unsigned* ctr = &st->wctr[ps];
+    unsigned* ctr = &st->ctl[1].wctr[ps];
     ps = ps == 2 ? 0 : ps + 1;
-    if (leader) st->wctr[ps] = 0u;
+    if (leader) st->ctl[1].wctr[ps] = 0u;
     // Unit size of the rows pushed for a seeding phase of about `items` work
     // items, and of the loop's rows.
     auto units_for = [&](unsigned items) { return unit_slots_for(items, E.nwarps, p.unit_slots); };
@@ -2351,9 +2351,9 @@ __global__ void __launch_bounds__(kThreads, 2) init_color_kernel(const __grid_co
   const int CH = p.unit_slots;
   int ps = 0;
   auto ctr = [&]() -> unsigned* {
-    unsigned* c = &st->wctr[ps];
+    unsigned* c = &st->ctl[1].wctr[ps];
     ps = ps == 2 ? 0 : ps + 1;
-    if (leader) st->wctr[ps] = 0u;
+    if (leader) st->ctl[1].wctr[ps] = 0u;
     return c;
   };
   if (leader) st->t_recolor[0] = globaltimer_ns();
