@@ -115,6 +115,7 @@ dc_status ensure_recolor_scratch(dc_ctx* ctx) {
     if (ctx->opt.heavy_min_live > 0) {
       HriBufs& h = ctx->hri;
       if ((s = dalloc(ctx, &h.hid, n, "heavy-row ids")) != DC_OK) return s;
+      if (ctx->opt.variant == DC_HB && (s = dalloc(ctx, &ctx->c8, n, "byte colours")) != DC_OK) return s;
       if (ctx->opt.variant == DC_HI && (s = dalloc(ctx, &h.bmF, words, "changed-colour bitmap")) != DC_OK)
         return s;
     }
@@ -259,6 +260,7 @@ RecolorParams recolor_params(dc_ctx* ctx, const dc_change* ch, long long k) {
   p.mem_cap = ctx->mem_cap;
   p.mout = ctx->mout;
   p.cp = ctx->cp;
+  p.c8 = ctx->c8;
   p.hri = ctx->hri;
   p.lflag = ctx->lflag;
   if (ctx->ngraphs > 0) {
@@ -702,6 +704,7 @@ void dc_destroy(dc_ctx* ctx) {
   dfree(ctx, &ctx->mem);
   dfree(ctx, &ctx->mout);
   dfree(ctx, &ctx->cp);
+  dfree(ctx, &ctx->c8);
   dfree(ctx, &ctx->hri.hid);
   dfree(ctx, &ctx->hri.bmF);
   dfree(ctx, &ctx->hri.hrow);

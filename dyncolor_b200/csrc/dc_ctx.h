@@ -63,6 +63,7 @@ struct dc_ctx {
   int* mem = nullptr;      // frontier member list of the recolour loop
   long long mem_cap = 0;
   int* mout = nullptr;     // members the loop's commit touches
+  unsigned char* c8 = nullptr;       // HB, with the index: byte colours
   unsigned long long* cp = nullptr;  // HB: packed (degree property, colour) per vertex
   HriBufs hri{};                     // HI: heavy-row index (min_live 0: off)
 

@@ -229,6 +229,7 @@ struct RecolorParams {
   long long mem_cap;
   int* mout;             // n: the iteration's members that leave
   unsigned long long* cp;  // HB: n packed (degree property, colour) words
+  unsigned char* c8;       // HB, with the index: n byte colours
   HriBufs hri;             // HI: heavy-row index (hri.min_live == 0: off)
   unsigned char* lflag;  // k
   int* pred;             // initial colouring: neighbours still to be coloured before each vertex

@@ -89,6 +89,9 @@ struct Env {
   // HB: (degree property << 32) | colour word per vertex, so one 8-byte
   // gather gives both; the frontier flags live in its colour half
   unsigned long long* cp;
+  // HB, with the index: each vertex's colour, those of kC8Top or more as
+  // kC8Top, for the walks of indexed rows, which need nothing else
+  unsigned char* c8;
   HriBufs hri;       // heavy-row index
   bool hri_on;       // HI: index in use
   bool hri_split;    // HB: indexed rows list their prior neighbours first
@@ -597,8 +600,12 @@ __device__ __forceinline__ bool merge_masks(unsigned* gm, unsigned* sm, int nw, 
   return true;
 }
 
+constexpr int kC8Top = 255;
+__device__ __forceinline__ unsigned char to_c8(int c) { return (unsigned char)min(c, kC8Top); }
+
 // Window bits of the colours at ids[e0..e1): four gathers in flight per
-// lane.
+// lane (HB: of the byte colours).
+template <int V>
 __device__ __forceinline__ void mask_colors(const Env& E, unsigned* sm, const int* ids, long long e0, long long e1,
                                             int nbits) {
   unsigned long long lm = 0;
@@ -611,7 +618,15 @@ __device__ __forceinline__ void mask_colors(const Env& E, unsigned* sm, const in
       cc[j] = idx < e1 ? ids[idx] : -1;
     }
 #pragma unroll
-    for (int j = 0; j < 4; ++j) cc[j] = cc[j] >= 0 ? (E.g.color[cc[j]] & kColorMask) : -1;
+    for (int j = 0; j < 4; ++j) {
+      const int u = cc[j];
+      if (V == DC_HB) {
+        cc[j] = u >= 0 ? (int)E.c8[u] : -1;
+        if (cc[j] == kC8Top) cc[j] = E.g.color[u];
+      } else {
+        cc[j] = u >= 0 ? (E.g.color[u] & kColorMask) : -1;
+      }
+    }
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int c = cc[j];
@@ -654,7 +669,7 @@ __device__ __noinline__ bool reduce_heavy(const unsigned* gmask, int4 un, int* o
   const int us = unit_span(xc, nch);
   const long long e0 = (long long)un.y * us;
   const long long e1 = min((long long)xc, e0 + us);
-  mask_colors(E, sm, H.xv + xb, e0, e1, nw * 32);
+  mask_colors<DC_HI>(E, sm, H.xv + xb, e0, e1, nw * 32);
   if (lane_id() == 0 && e1 > e0) sh.idx_reads[warp_id()] += e1 - e0;
   if (nch > 1 && !merge_masks(const_cast<unsigned*>(gmask) + un.z, sm, nw, nch)) return true;
   const int* cnt = H.hist + (long long)hi * kHriBins;
@@ -703,7 +718,7 @@ __device__ __noinline__ bool reduce_split(int4 un, bool loop, int* out) {
 #pragma unroll 1
   for (int k = lane_id(); k < nw; k += 32) sm[k] = 0;
   __syncwarp();
-  mask_colors(E, sm, H.ids + pb, 0, nh, nw * 32);
+  mask_colors<DC_HB>(E, sm, H.ids + pb, 0, nh, nw * 32);
   int r = first_zero(sm, nw);
   __syncwarp();
   if (r < 0) r = slow_mex(v, M_MEX_PRIOR, kMaskBits);  // every colour of the window present
@@ -1003,6 +1018,63 @@ __device__ __forceinline__ void push4(const Env& E, Target T, const Rule* R, con
   }
 }
 
+// HB: dirty marks of an indexed row's changed vertex that marks no one (it
+// was a member before its last commit), over ids[lo..top) of the neighbours
+// behind it.  Nine in ten entries fail the test on the colour, and nearly all
+// that pass are dirty already, so the walk is its gathers, and these are
+// bound by the cache lines a warp's 32 lanes touch (one a clock per SM; about
+// 23 of 128 vertices each at R-MAT scale 22).  Byte colours need fewer and
+// more often hit the L1 than the packed words: 62 M entries in 190 us where
+// the packed words took 219, the whole batch 80.0 -> 75.7 ms.  (Ordering the
+// rows by launch-start colour leaves 17 % of the entries, but with change
+// lists that hold most neighbours after 20 iterations nothing is saved;
+// ordering them by how many neighbours come before each, which bounds its
+// colour, leaves 80 %.)
+__device__ __noinline__ void push_dirty(Target T, const int* ids, int lo, int top, int pv, int cv) {
+  const Env& E = env();
+  const unsigned char* c8 = E.c8;
+  constexpr int U = 4;
+  int nx[U];
+#pragma unroll
+  for (int j = 0; j < U; ++j) {
+    const int i = lo + j * 32 + lane_id();
+    nx[j] = i < top ? __ldcg(ids + i) : -1;
+  }
+#pragma unroll 1
+  for (int r0 = lo; r0 < top; r0 += 32 * U) {
+    int uu[U], cc[U];
+    bool any = false;
+#pragma unroll
+    for (int j = 0; j < U; ++j) {
+      uu[j] = nx[j];
+      const int i = r0 + 32 * U + j * 32 + lane_id();
+      nx[j] = i < top ? __ldcg(ids + i) : -1;
+    }
+#pragma unroll
+    for (int j = 0; j < U; ++j) cc[j] = uu[j] >= 0 ? (int)c8[uu[j]] : -1;
+#pragma unroll
+    for (int j = 0; j < U; ++j) {
+      if (uu[j] < 0 || !(cc[j] > pv || cc[j] == cv || cc[j] == kC8Top)) uu[j] = -1;
+      any |= uu[j] >= 0;
+    }
+    if (!__any_sync(0xffffffffu, any)) continue;
+    unsigned cw[U];
+#pragma unroll
+    for (int j = 0; j < U; ++j) cw[j] = uu[j] >= 0 ? E.clean[uu[j] >> 5] : 0u;
+#pragma unroll
+    for (int j = 0; j < U; ++j) {
+      const unsigned bit = 1u << (uu[j] & 31);
+      if (!(cw[j] & bit)) continue;
+      if (cc[j] == kC8Top) {
+        const int cu = E.g.color[uu[j]];
+        if (!(pv < cu || cv == cu)) continue;
+      }
+      if (atomicAnd(&E.clean[uu[j] >> 5], ~bit) & bit) stage_eval(E, T, uu[j]);
+    }
+    __syncwarp();
+  }
+}
+
 // PUSH over piece `sub` of `pieces` of one unit of a row: its neighbours, or,
 // of an indexed row, HI: the parts of its ordered copy and its change list
 // that push_parts named; HB: the part of its copy behind the prior
@@ -1045,6 +1117,11 @@ __device__ __noinline__ void push_unit(Target T, int4 un, const unsigned* gmask,
   const int us = unit_span(n, un.w * pieces), piece = un.y * pieces + sub;
   const int lo = piece * us;
   const int top = piece == un.w * pieces - 1 ? total : min(total, lo + us);
+  if (V == DC_HB && indexed && !(R[0].pv & kNewBit)) {
+    if (R[0].pv != R[0].cv) push_dirty(T, ids, lo, top, R[0].pv, R[0].cv);
+    if (lane_id() == 0 && lo < top) sh.idx_reads[warp_id()] += top - lo;
+    return;
+  }
   const int np = P.x + P.z;  // entries in the ordered copy
   const int* color = E.g.color;
   // the ids of round r0 + 128 are loaded before round r0's are consumed
@@ -1660,6 +1737,7 @@ __device__ __noinline__ void phase_commit(Target T, int it, int ring) {
     if (nc != oc) {
       if (V == DC_HB) {
         g.color[v] = nc;
+        if (E.hri_split) E.c8[v] = to_c8(nc);
         if (E.gchg) atomicAdd(&E.gchg[E.gid[v]], 1);
       } else if (E.hri_on && mark_bit(E.hri.bmF, v)) {
         push_first(v, oc);
@@ -1756,6 +1834,7 @@ __device__ __noinline__ void phase_seed_commit(int buf, int q, int kind, int ch)
     g.prev[v] = V == DC_HB ? (oc | kNewBit) : oc;
     g.color[v] = nc;
     if (V == DC_HB) *flag_word<V>(E, v) = (unsigned)nc;
+    if (V == DC_HB && E.hri_split) E.c8[v] = to_c8(nc);
     // first colour change since the heavy-row index was built
     if (V == DC_HI && E.hri_on && nc != oc && mark_bit(E.hri.bmF, v)) push_first(v, oc);
     cmax_local = max(cmax_local, nc);
@@ -1901,6 +1980,7 @@ __device__ __forceinline__ void setup_env(const RecolorParams& p) {
     E.bmA = p.bmA;
     E.ncolor = p.ncolor;
     E.cp = p.cp;
+    E.c8 = p.c8;
     E.hri = p.hri;
     E.hri_on = E.hri_split = false;
     E.mem = p.mem;
@@ -1999,8 +2079,11 @@ __global__ void __launch_bounds__(kThreads, 2) recolor_kernel(const __grid_const
         // packed (degree property, colour) words for this launch's gathers;
         // this phase's barrier publishes them
 #pragma unroll 1
-        for (long long v = gtid; v < p.g.n; v += gthreads)
-          p.cp[v] = ((unsigned long long)(unsigned)p.g.prop[v] << 32) | (unsigned)(p.g.color[v] & kColorMask);
+        for (long long v = gtid; v < p.g.n; v += gthreads) {
+          const int c = p.g.color[v] & kColorMask;
+          p.cp[v] = ((unsigned long long)(unsigned)p.g.prop[v] << 32) | (unsigned)c;
+          if (E.hri_split) p.c8[v] = to_c8(c);
+        }
         phase_lines<V>(ph, p.ch, K, p.lflag, units_for((unsigned)(K / 16)));
         break;
       case P_D1: case P_I1: case P_I3:

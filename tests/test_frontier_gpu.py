@@ -80,3 +80,37 @@ def test_improper_start_and_repeated_batches(variant, ov):
         assert (sg.iterations, sg.seed_targets, sg.frontier_total) == (
             so.iterations, so.seed_targets, so.frontier_total)
     ctx.close()
+
+
+@pytest.mark.parametrize("variant,ov", [(dc.HI, po.HI), (dc.HB, po.HB)])
+@pytest.mark.parametrize("clique", [250, 255, 256, 257, 300])
+def test_colours_past_one_byte_in_indexed_rows(variant, ov, clique):
+    """A clique with as many colours as vertices, hung with leaves so that its
+    rows are indexed and reach behind it: walks of indexed rows that keep one
+    byte per colour must still tell colours above it apart."""
+    rng = np.random.default_rng(clique)
+    n = clique + 1500
+    x, y = np.triu_indices(clique, 1)
+    lx, ly = rng.integers(0, clique, 12000), rng.integers(clique, n, 12000)
+    a = np.concatenate([x, lx, clique + np.arange(1499)]).astype(np.int32)
+    b = np.concatenate([y, ly, clique + 1 + np.arange(1499)]).astype(np.int32)
+    a, b = dc.dedup(n, a, b)
+    col = dc.greedy_color(n, a, b)
+    assert col.max() >= clique - 1
+    ctx = dc.Context(variant=variant, heavy_min_live=64)
+    ctx.load_edges(n, a, b)
+    ctx.set_colors(col)
+    g = oracle_graph(n, a, b, col)
+    for i in range(5):
+        # edges inside the clique go and come back, and some of the leaves'
+        p, q = rng.integers(0, clique, 200), rng.integers(0, clique, 200)
+        r, s = rng.integers(0, clique, 200), rng.integers(clique, n, 200)
+        u, v = np.concatenate([p, r]), np.concatenate([q, s])
+        keep = u != v
+        ch = po.as_changes(u[keep], v[keep], rng.integers(0, 2, keep.sum()))
+        rc, so = g.apply_batch(ch, ov, po.SNAPSHOT)
+        sg = ctx.apply_batch(to_dc_changes(ch))
+        assert rc == po.OK and np.array_equal(ctx.colors(), g.colors())
+        assert (sg.iterations, sg.seed_targets, sg.frontier_total) == (
+            so.iterations, so.seed_targets, so.frontier_total)
+    ctx.close()
