@@ -1545,9 +1545,13 @@ __device__ __noinline__ void phase_mark(Target T, int it, int ring, bool push, b
   const unsigned per = (len + free - 1) / free;
   const unsigned m = per < 1 ? 1 : per < 32 ? per : 32 * W;
   const unsigned nP = (len + m - 1) / m;
-  // entries of a long row searched inline: most searches that succeed do so
-  // early, but a warp's searches come one after another
-  const int inl = m == 1 ? 512 : 128;
+  // Entries of a long row searched inline; the rest goes on beside the next
+  // phase's mexes, a piece per warp.  Each 128 are a chain of three dependent
+  // loads, and HI's searches mostly go on to the end of the row: none inline
+  // took R-MAT scale 24 from 85.5 to 81.4 ms a batch and scale 16 from 3.37
+  // to 2.92 against 512 for a member that has its warp alone and 128 else.
+  // HB's end early (2 in 3 within 128; none inline is 2 % slower at scale 16).
+  const int inl = V == DC_HI ? 0 : 128;
   const unsigned rows = batch_rows(cA, nU + nP, E.nwarps);
   Grabber gb(ctr, nU + nP + (cA + rows - 1) / rows, team_warp(), E.nwarps);
   unsigned i;
