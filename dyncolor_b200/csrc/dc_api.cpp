@@ -65,7 +65,11 @@ dc_status ensure_recolor_scratch(dc_ctx* ctx) {
     QueueBufs& q = ctx->qb[b];
     if ((s = dalloc(ctx, &q.itemsA, n, "queue items")) != DC_OK) return s;
     if ((s = dalloc(ctx, &q.units, capU, "queue units")) != DC_OK) return s;
-    const long long capM = b == 2 ? capM_dist : capM_mex;
+    // buffer 1 also holds SCAN's rows (any longer than kScanBatch), buffer 0
+    // the pushing rows that have their index's colour starts
+    const long long capM = b == 2   ? capM_dist
+                           : b == 1 ? capM_mex + kScanWords * std::min<long long>(n, ctx->pool_cap / kScanBatch)
+                                    : capM_mex + kPushWords * std::min<long long>(n, kCapHist);
     if ((s = dalloc(ctx, &q.gmask, capM, "queue masks")) != DC_OK) return s;
     q.capA = n;
     q.capU = capU;
@@ -83,7 +87,7 @@ dc_status ensure_recolor_scratch(dc_ctx* ctx) {
     h.cap_pairs = hi ? ctx->pool_cap / 4 + 4096 : ctx->pool_cap / 2 + 8192;
     h.cap_exc = hi ? h.cap_pairs : 1;       // a row's change list holds at most its live neighbours
     h.cap_a = hi ? n / 8 + ctx->pool_cap / 512 + 1024 : 1;  // items of 512 slots
-    h.cap_hist = hi ? std::min<long long>(h.cap_rows, 1ll << 16) : 0;
+    h.cap_hist = hi ? std::min<long long>(h.cap_rows, kCapHist) : 0;
     if ((s = dalloc(ctx, &h.hrow, h.cap_rows, "heavy rows")) != DC_OK) return s;
     if ((s = dalloc(ctx, &h.hoff, h.cap_rows + 1, "heavy-row offsets")) != DC_OK) return s;
     if ((s = dalloc(ctx, &h.xoff, h.cap_rows + 1, "change-list offsets")) != DC_OK) return s;

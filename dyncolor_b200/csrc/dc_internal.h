@@ -35,6 +35,10 @@ constexpr int kNumQueues = 8;       // logical queue counter slots
 constexpr long long kMemSlack = 4096;     // member-list entries the loop may add beyond half the live ones before a rebuild
 constexpr int kUnitSlotsDefault = 4096;  // adjacency slots per warp work unit
 constexpr int kLoopUnit = 512;           // slots per work unit of the recolour loop's rows, at most
+constexpr int kScanBatch = 32;           // witness searches up to this length are taken 32 rows at a time
+constexpr int kScanWords = 4;            // mask region of a longer one that goes on in units
+constexpr int kPushWords = 12;           // mask region of a pushing indexed row (the last five fields of its plan)
+constexpr int kCapHist = 1 << 16;        // indexed rows that keep their colour counts and starts, at most
 constexpr long long kLoadPiece = 1ll << 27;  // edge pairs per structural launch of a graph load
 constexpr int kBarrierTimeoutMsDefault = 20000;  // grid-barrier wait limit unless the options set one
 
@@ -64,7 +68,7 @@ struct LoopState {
   unsigned a_count;      // (vertex, chunk) items waiting for the append phase
   unsigned m_rebuild[3]; // 1: rebuild the member list before the iteration
   int chg[3];            // "a colour changed" flags
-  unsigned pad;
+  unsigned hri_off;      // 1: the index is incomplete for this batch; full scans only
 };
 
 // Grid barrier and work-grab counters of one cooperative launch.
@@ -110,8 +114,6 @@ struct DevState {
   unsigned long long phase_ns[6];     // recolour launch: seeding, find-eligible, mex, commit, 2 spare
   // heavy-row index
   unsigned long long hcount;          // rows found with at least min_live live slots
-  unsigned hri_off;                   // 1: the index is incomplete for this batch; full scans only
-  unsigned pad1;
 };
 
 struct GraphDev {

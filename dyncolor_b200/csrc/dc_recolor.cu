@@ -281,8 +281,8 @@ __device__ __noinline__ void write_row(Target T, int u, int L, Plan P, unsigned 
   int ms = -1;
   if (T.mode == R_PUSH) {
     if (P.parts.x >= 0) {
-      const unsigned mo = atomicAdd(&qc->masks, 4u);
-      if ((long long)mo + 4 > qb.capM) {
+      const unsigned mo = atomicAdd(&qc->masks, (unsigned)kPushWords);
+      if ((long long)mo + kPushWords > qb.capM) {
         atomicOr(status, ST_OVERFLOW);
         return;
       }
@@ -305,7 +305,7 @@ __device__ __forceinline__ int4 push_parts(const Env& E, int v) {
   const HriBufs& H = E.hri;
   const int hi = H.hid[v];
   int4 P = make_int4(-1, 0, 0, 0);
-  if (hi < 0 || hi >= H.cap_hist || ld_cg(&E.st->hri_off) != 0u) return P;
+  if (hi < 0 || hi >= H.cap_hist || inputs().hri_off != 0u) return P;
   const int xc = ld_cg(&H.xcnt[hi]);
   if ((long long)xc > H.xoff[hi + 1] - H.xoff[hi]) return P;  // its change list is incomplete
   const int* start = H.hstart + (long long)hi * kHriBins;  // entries above each colour (top bin: 0)
@@ -331,7 +331,7 @@ __device__ __forceinline__ int indexed_len(const Env& E, int u) {
   if (E.hri_split) return H.hid[u] >= 0 ? 1 : -1;
   if (!E.hri_on) return -1;
   const int hi = H.hid[u];
-  if (hi < 0 || hi >= H.cap_hist || ld_cg(&E.st->hri_off) != 0u) return -1;
+  if (hi < 0 || hi >= H.cap_hist || inputs().hri_off != 0u) return -1;
   const int xc = ld_cg(&H.xcnt[hi]);
   return (long long)xc > H.xoff[hi + 1] - H.xoff[hi] ? -1 : xc;  // longer: the list overflowed
 }
@@ -1096,7 +1096,7 @@ __device__ __noinline__ void push_unit(Target T, int4 un, const unsigned* gmask,
   Rule R[4];
   R[0] = R[1] = R[2] = R[3] = rule_of<V>(E, v);
   int total = L;
-  if (V == DC_HI && un.z >= 0 && ld_cg(&E.st->hri_off) == 0u) {
+  if (V == DC_HI && un.z >= 0 && inputs().hri_off == 0u) {
     indexed = true;
     P = ld_cg(reinterpret_cast<const int4*>(gmask + un.z));
     const int hi = E.hri.hid[v];
@@ -1216,7 +1216,6 @@ __device__ __noinline__ void push_batchA(Target T, const int* items, unsigned cA
 // ---------------------------------------------------------------------
 // PULL: which members stay
 // ---------------------------------------------------------------------
-constexpr int kScanBatch = 32;    // failing rows up to this length are searched 32 rows at a time
 constexpr int kScanUnit = 512;    // longer rows than a warp searches inline go on in units of this
 
 
@@ -1328,9 +1327,9 @@ __device__ __noinline__ void push_scan(int u, int from, int len, unsigned at) {
   const QueueBufs& sq = E.qb[1];
   QCount* sc = &E.ls->q[Q_SCAN];
   const int c = (len - from + kScanUnit - 1) / kScanUnit;
-  const unsigned mo = atomicAdd(&sc->masks, 4u);
+  const unsigned mo = atomicAdd(&sc->masks, (unsigned)kScanWords);
   const unsigned pu = atomicAdd(&sc->countU, (unsigned)c);
-  if ((long long)mo + 4 > sq.capM) {
+  if ((long long)mo + kScanWords > sq.capM) {
     atomicOr(&E.st->status, ST_OVERFLOW);
     return;
   }
@@ -1634,7 +1633,7 @@ __device__ __noinline__ void push_first(int v, int c0) {
   if (c == 0) return;
   const unsigned b = atomicAdd(&E.ls->a_count, (unsigned)c);
   if ((long long)b + c > E.hri.cap_a) {
-    atomicExch(&E.st->hri_off, 1u);
+    atomicExch(&E.ls->hri_off, 1u);
     return;
   }
   const int bin = c0 < kHriBins - 1 ? c0 : kHriBins - 1;
@@ -1650,7 +1649,7 @@ __device__ __noinline__ void phase_append(unsigned* ctr) {
   const Env& E = env();
   const HriBufs& H = E.hri;
   // an overflowed queue has unwritten items, and the index is off anyway
-  if (ld_cg(&E.st->hri_off) != 0u) return;
+  if (inputs().hri_off != 0u) return;
   Grabber gb(ctr, (unsigned)min((long long)inputs().a_count, H.cap_a), team_warp(), E.nwarps);
   unsigned i;
 #pragma unroll 1

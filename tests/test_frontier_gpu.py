@@ -114,3 +114,32 @@ def test_colours_past_one_byte_in_indexed_rows(variant, ov, clique):
         assert (sg.iterations, sg.seed_targets, sg.frontier_total) == (
             so.iterations, so.seed_targets, so.frontier_total)
     ctx.close()
+
+
+@pytest.mark.parametrize("variant,ov", [(dc.HI, po.HI), (dc.HB, po.HB)])
+@pytest.mark.parametrize("degree", [32, 34, 40])
+def test_every_row_just_past_the_short_search(variant, ov, degree):
+    """A ring lattice whose rows all end just past the length up to which
+    witness searches run 32 rows at a time, with a first frontier of nearly
+    every vertex: each search that goes on takes a region of its own."""
+    rng = np.random.default_rng(degree)
+    n = 20000
+    v = np.arange(n, dtype=np.int32)
+    a = np.concatenate([v] * (degree // 2))
+    b = np.concatenate([(v + k + 1) % n for k in range(degree // 2)]).astype(np.int32)
+    a, b = dc.dedup(n, a, b)
+    col = rng.integers(0, degree, n).astype(np.int32)
+    ctx = dc.Context(variant=variant, slack=1.01)
+    ctx.load_edges(n, a, b)
+    ctx.set_colors(col)
+    g = oracle_graph(n, a, b, col)
+    for i in range(2):
+        x = rng.integers(0, n, 30000)
+        y = (x + 1 + rng.integers(0, degree // 2, 30000)) % n
+        ch = po.as_changes(x, y, rng.integers(0, 2, 30000))
+        rc, so = g.apply_batch(ch, ov, po.SNAPSHOT)
+        sg = ctx.apply_batch(to_dc_changes(ch))
+        assert rc == po.OK and np.array_equal(ctx.colors(), g.colors())
+        assert (sg.iterations, sg.seed_targets, sg.frontier_total) == (
+            so.iterations, so.seed_targets, so.frontier_total)
+    ctx.close()
