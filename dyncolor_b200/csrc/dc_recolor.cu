@@ -83,6 +83,7 @@ struct Env {
   DevState* st;
   LoopState* ls;     // the loop's counters
   unsigned nwarps;   // warps of the grid
+  int loop_units;    // slots per work unit of the loop's rows
   QueueBufs qb[3];
   unsigned* bmA;
   int* ncolor;
@@ -120,6 +121,22 @@ struct Rows {
   int a[32], b[32], c[32], d[32];
 };
 
+// Where a launch is in its sequence of phases.
+struct Step {
+  int ph;         // the phase
+  int ps;         // phase count mod 3, for the ring of work counters
+  int r, rn;      // it % 3, (it + 1) % 3
+  long long it;   // the loop's iteration
+};
+
+// The work items of a MARK or EVAL phase: units in 2^us pieces, then (MARK)
+// shares of 2^ms members, then class-A batches of 2^as rows.
+struct Work {
+  unsigned units, members, total;  // items of the first kind, of the first two, of all
+  int us, ms, as;
+  int sh;                          // log2 of the items a warp takes at a time
+};
+
 struct Shared {
   Env E;
   LoopState snap;                     // the loop's counters at the last grid barrier
@@ -136,6 +153,8 @@ struct Shared {
   unsigned qn[2], qbase[4];           // the CTA's bulk push: items and units, queue, row-list and member positions
   int ok;                             // the last grid barrier did not time out
   unsigned bar;                       // arrivals the last grid barrier waited for
+  Step step;                          // what the CTA does next
+  Work work;
   // CTA 0 thread 0: time per phase kind, the time of the last lap, the
   // frontier sizes' sum, member-list entries in vertex order
   unsigned long long acc[4], t_last;
@@ -161,29 +180,48 @@ __device__ __forceinline__ unsigned grab(unsigned* ctr) {
   return __shfl_sync(0xffffffffu, x, 0);
 }
 
+// Smallest s <= top for which `warps` warps with 2^s of the items each take
+// them all.  Shares are powers of two, found without a division.
+__device__ __forceinline__ int share(unsigned items, unsigned warps, int top) {
+  int s = 0;
+  while (s < top && (warps << s) < items) ++s;
+  return s;
+}
+
 // Hands out the work items [0, total) of a phase to warps.  Every warp's
-// first `per` items follow from its own number; the rest are taken `per` at
+// first 2^sh items follow from its own number; the rest are taken 2^sh at
 // a time from the phase's counter (a counter takes one atomic at a time, so
 // one item per atomic would bound a phase of hundreds of thousands of
-// items).  `per` grows with the items per warp (at most 32), keeping the
+// items).  2^sh grows with the items per warp (at most 32), keeping the
 // tail imbalance small.  A phase of no more items than warps uses no atomic.
+__device__ __forceinline__ int grab_share(unsigned items, unsigned warps) {
+  int s = 0;
+  while (s < 5 && (16u * warps << s) <= items) ++s;
+  return s;
+}
 struct Grabber {
   unsigned* ctr;  // nullptr: no counter, the warps take their items in turn
-  unsigned total, per, cur, end, base, step;
+  unsigned total, cur, end, base, step;
+  int sh;
   __device__ __forceinline__ Grabber(unsigned* c, unsigned t, unsigned gwarp, unsigned nwarps) : ctr(c), total(t) {
-    per = t / (8 * nwarps);
-    per = per < 1 ? 1 : (per > 32 ? 32 : per);
-    step = nwarps * per;
-    base = gwarp * per;
+    start(grab_share(t, nwarps), gwarp, nwarps);
+  }
+  __device__ __forceinline__ Grabber(unsigned* c, const Work& w, unsigned gwarp, unsigned nwarps) : ctr(c), total(w.total) {
+    start(w.sh, gwarp, nwarps);
+  }
+  __device__ __forceinline__ void start(int s, unsigned gwarp, unsigned nwarps) {
+    sh = s;
+    step = nwarps << sh;
+    base = gwarp << sh;
     cur = base;
-    end = min(total, cur + per);
+    end = min(total, cur + (1u << sh));
   }
   // Warp-uniform.
   __device__ __forceinline__ bool next(unsigned& i) {
     if (cur >= end) {
       if (step >= total) return false;
       if (ctr) {
-        cur = step + grab(ctr) * per;
+        cur = step + (grab(ctr) << sh);
       } else {
         base += step;
         cur = base;
@@ -192,7 +230,7 @@ struct Grabber {
         end = cur;
         return false;
       }
-      end = min(total, cur + per);
+      end = min(total, cur + (1u << sh));
     }
     i = cur++;
     return true;
@@ -885,20 +923,18 @@ __device__ __noinline__ void reduce_batchA(const int* items, unsigned cA, unsign
 // that leaves warps without work (a batch of 32 rows of 32 slots is eight
 // dependent rounds for its warp, one of four rows is one).  Lanes past the
 // batch's rows get an index past the queue.
-__device__ __forceinline__ unsigned batch_rows(unsigned cA, unsigned cU, unsigned nwarps) {
-  const unsigned free = nwarps > 2 * cU ? nwarps - cU : nwarps / 2;
-  const unsigned per = (cA + free - 1) / free;
-  return per < 1 ? 1 : per > 32 ? 32 : per;
+__device__ __forceinline__ int batch_share(unsigned cA, unsigned cU, unsigned nwarps) {
+  return share(cA, nwarps > 2 * cU ? nwarps - cU : nwarps / 2, 5);
 }
+__device__ __forceinline__ unsigned shares(unsigned items, int s) { return (items + (1u << s) - 1) >> s; }
 // Pieces a phase's units are walked in: a unit of the loop is kLoopUnit slots
-// (kPieces rounds of a warp's walk); while there are idle warps, each round
+// (four rounds of a warp's walk); while there are idle warps, each round
 // gets a warp of its own.
-constexpr unsigned kPieces = 4;
-__device__ __forceinline__ unsigned unit_pieces(unsigned units, unsigned nwarps) {
-  return units <= nwarps / 2 ? kPieces : units <= nwarps ? 2 : 1;
+__device__ __forceinline__ int unit_pieces(unsigned units, unsigned nwarps) {  // log2
+  return units <= nwarps / 2 ? 2 : units <= nwarps ? 1 : 0;
 }
-__device__ __forceinline__ unsigned batch_item(unsigned b, unsigned per) {
-  return lane_id() < (int)per ? b * per + lane_id() : 0xffffffffu;
+__device__ __forceinline__ unsigned batch_item(unsigned b, int s) {
+  return lane_id() < (1 << s) ? (b << s) + lane_id() : 0xffffffffu;
 }
 
 template <int V>
@@ -908,8 +944,8 @@ __device__ __noinline__ void phase_reduce(int buf, int q, unsigned* ctr, int mod
   const QCount& qc = inputs().q[q];
   const unsigned cA = (unsigned)min((long long)qc.countA, qb.capA);
   const unsigned cU = (unsigned)min((long long)qc.countU, qb.capU);
-  const unsigned per = batch_rows(cA, cU, E.nwarps);
-  Grabber gb(ctr, cU + (cA + per - 1) / per, team_warp(), E.nwarps);
+  const int per = batch_share(cA, cU, E.nwarps);
+  Grabber gb(ctr, cU + shares(cA, per), team_warp(), E.nwarps);
   unsigned i;
 #pragma unroll 1
   while (gb.next(i)) {
@@ -1527,41 +1563,31 @@ __device__ __noinline__ void pull_members(Target T, int it, int ring, unsigned b
 // marks; HI's first iteration pushes first, because its members have no
 // witnesses yet and all of them push).
 template <int V>
-__device__ __noinline__ void phase_mark(Target T, int it, int ring, bool push, bool pull, unsigned* ctr) {
+__device__ __noinline__ void phase_mark(Target T, int it, int ring, unsigned* ctr) {
   constexpr unsigned W = V == DC_HB ? 4 : 2;
   const Env& E = env();
   const LoopState& in = inputs();
-  const QueueBufs& fq = E.qb[0];
-  const QCount& fc = in.q[Q_PUSH];
-  const unsigned cA = push ? (unsigned)min((long long)fc.countA, fq.capA) : 0;
-  const unsigned cU = push ? (unsigned)min((long long)fc.countU, fq.capU) : 0;
-  const unsigned len = pull ? (unsigned)min((long long)in.m_len[ring], E.mem_cap) : 0;
-  // units go in up to kPieces pieces while there are warps for them; a short
-  // member list is spread over the warps left
-  const unsigned pieces = unit_pieces(cU, E.nwarps);
-  const unsigned nU = cU * pieces;
-  const unsigned free = E.nwarps > 2 * nU ? E.nwarps - nU : E.nwarps / 2;
-  const unsigned per = (len + free - 1) / free;
-  const unsigned m = per < 1 ? 1 : per < 32 ? per : 32 * W;
-  const unsigned nP = (len + m - 1) / m;
-  // Entries of a long row searched inline; the rest goes on beside the next
-  // phase's mexes, a piece per warp.  Each 128 are a chain of three dependent
-  // loads, and HI's searches mostly go on to the end of the row: none inline
-  // took R-MAT scale 24 from 85.5 to 81.4 ms a batch and scale 16 from 3.37
-  // to 2.92 against 512 for a member that has its warp alone and 128 else.
-  // HB's end early (2 in 3 within 128; none inline is 2 % slower at scale 16).
-  const int inl = V == DC_HI ? 0 : 128;
-  const unsigned rows = batch_rows(cA, nU + nP, E.nwarps);
-  Grabber gb(ctr, nU + nP + (cA + rows - 1) / rows, team_warp(), E.nwarps);
+  const Work& w = shared().work;
+  Grabber gb(ctr, w, team_warp(), E.nwarps);
   unsigned i;
 #pragma unroll 1
   while (gb.next(i)) {
-    if (i < nU)
-      push_unit<V>(T, fq.units[i / pieces], fq.gmask, (int)(i % pieces), (int)pieces);
-    else if (i < nU + nP)
-      pull_members<V, W>(T, it, ring, (i - nU) * m, m, len, inl);
-    else
-      push_batchA<V>(T, fq.itemsA, cA, batch_item(i - nU - nP, rows));
+    if (i < w.units) {
+      push_unit<V>(T, E.qb[0].units[i >> w.us], E.qb[0].gmask, (int)(i & ((1u << w.us) - 1)), 1 << w.us);
+    } else if (i < w.members) {
+      // Entries of a long row searched inline; the rest goes on beside the
+      // next phase's mexes, a piece per warp.  Each 128 are a chain of three
+      // dependent loads, and HI's searches mostly go on to the end of the
+      // row: none inline took R-MAT scale 24 from 85.5 to 81.4 ms a batch and
+      // scale 16 from 3.37 to 2.92 against 512 for a member that has its warp
+      // alone and 128 else.  HB's end early (2 in 3 within 128; none inline
+      // is 2 % slower at scale 16).
+      pull_members<V, W>(T, it, ring, (i - w.units) << w.ms, 1u << w.ms,
+                         (unsigned)min((long long)in.m_len[ring], E.mem_cap), V == DC_HI ? 0 : 128);
+    } else {
+      push_batchA<V>(T, E.qb[0].itemsA, (unsigned)min((long long)in.q[Q_PUSH].countA, E.qb[0].capA),
+                     batch_item(i - w.members, w.as));
+    }
   }
   finish_push(T);
 }
@@ -1569,20 +1595,20 @@ __device__ __noinline__ void phase_mark(Target T, int it, int ring, bool push, b
 // SCAN over one piece of a unit: nothing to look for once another piece of
 // the row has a hit; the row's last piece settles the member.
 template <int V>
-__device__ __noinline__ void scan_piece(Target T, int it, int ring, int4 un, unsigned* gm, int sub, int pieces) {
+__device__ __noinline__ void scan_piece(Target T, int it, int ring, int4 un, unsigned* gm, int sub, int ps) {
   const Env& E = env();
   const int u = un.x;
   const uint4 head = ld_cg(reinterpret_cast<const uint4*>(gm));
   const Span sp = span_of<V>(E, u);
   const int cu = (int)(*flag_word<V>(E, u) & (unsigned)kColorMask);
   const int pu = V == DC_HB ? E.g.prop[u] : 0;
-  const int size = kScanUnit / pieces;
+  const int size = kScanUnit >> ps;
   const int s_lo = (int)head.w + un.y * kScanUnit + sub * size, s_hi = min(sp.len, s_lo + size);
   if (head.y == 0u && scan_span<V>(sp.at, s_lo, s_hi, u, cu, pu, sp.prior) && lane_id() == 0) atomicExch(&gm[1], 1u);
   __threadfence();
   __syncwarp();
   int last = 0;
-  if (lane_id() == 0) last = atomicAdd(&gm[0], 1u) == (unsigned)(un.w * pieces) - 1u;
+  if (lane_id() == 0) last = atomicAdd(&gm[0], 1u) == (unsigned)(un.w << ps) - 1u;
   if (!__any_sync(0xffffffffu, last)) return;
   __threadfence();
   int oc = O_NONE;
@@ -1597,24 +1623,19 @@ __device__ __noinline__ void phase_eval(Target T, int it, int ring, unsigned* ct
   const LoopState& in = inputs();
   const QueueBufs& sq = E.qb[1];
   const QueueBufs& eq = E.qb[2];
-  const QCount& ec = in.q[Q_EVAL + ring];
-  const unsigned cS = (unsigned)min((long long)in.q[Q_SCAN].countU, sq.capU);
-  const unsigned cA = (unsigned)min((long long)ec.countA, eq.capA);
-  const unsigned cU = (unsigned)min((long long)ec.countU, eq.capU);
-  const unsigned pieces = unit_pieces(cS, E.nwarps);
-  const unsigned nS = cS * pieces;
-  const unsigned per = batch_rows(cA, nS + cU, E.nwarps);
-  Grabber gb(ctr, nS + cU + (cA + per - 1) / per, team_warp(), E.nwarps);
+  const Work& w = shared().work;
+  Grabber gb(ctr, w, team_warp(), E.nwarps);
   unsigned i;
 #pragma unroll 1
   while (gb.next(i)) {
-    if (i < nS) {
-      const int4 un = sq.units[i / pieces];
-      scan_piece<V>(T, it, ring, un, sq.gmask + un.z, (int)(i % pieces), (int)pieces);
-    } else if (i < nS + cU) {
-      reduce_unit<V>(eq.units[i - nS], eq.gmask, mode, true, out);
+    if (i < w.units) {
+      const int4 un = sq.units[i >> w.us];
+      scan_piece<V>(T, it, ring, un, sq.gmask + un.z, (int)(i & ((1u << w.us) - 1)), w.us);
+    } else if (i < w.members) {
+      reduce_unit<V>(eq.units[i - w.units], eq.gmask, mode, true, out);
     } else {
-      reduce_batchA<V>(eq.itemsA, cA, batch_item(i - nS - cU, per), true, out);
+      reduce_batchA<V>(eq.itemsA, (unsigned)min((long long)in.q[Q_EVAL + ring].countA, eq.capA),
+                       batch_item(i - w.members, w.as), true, out);
     }
   }
 }
@@ -1908,8 +1929,13 @@ constexpr int kStateWords = sizeof(LoopState) / 4;
 // The grid barrier, after which every CTA has a snapshot of the counters in
 // shared memory (one round trip for all of them).  Phases and decisions read
 // their inputs there; a counter that the phase under way changes may be
-// newer or older in it and is not read.
-__device__ __noinline__ bool sync_grid(DevState* st, unsigned long long timeout_ns) {
+// newer or older in it and is not read.  `decide` then runs in thread 0 alone:
+// the same few hundred instructions in 32 warps of every SM, cold in the
+// instruction caches, were 2.6 us of each phase (R-MAT 24: 82.7 -> 76.7 ms a
+// batch with this and the work of a phase planned here too, R-MAT 16 2.89 ->
+// 2.68).
+template <class F>
+__device__ __forceinline__ bool sync_grid(DevState* st, unsigned long long timeout_ns, F decide) {
   Shared& sh = shared();
   __syncthreads();
   if (warp_id() == 0) {
@@ -1920,9 +1946,156 @@ __device__ __noinline__ bool sync_grid(DevState* st, unsigned long long timeout_
       if (i + lane_id() < kStateWords)
         reinterpret_cast<unsigned*>(&sh.snap)[i + lane_id()] =
             ld_cg(reinterpret_cast<unsigned*>(&st->ls) + i + lane_id());
+    __syncwarp();
+    if (lane_id() == 0) decide();
   }
   __syncthreads();
   return sh.ok != 0;
+}
+__device__ __noinline__ bool sync_grid(DevState* st, unsigned long long timeout_ns) {
+  return sync_grid(st, timeout_ns, [] {});
+}
+
+// Phase timer: CTA 0 thread 0 reads %globaltimer after a barrier and charges
+// the time since the last lap to the phase kind that just ended.
+__device__ __forceinline__ void lap(int kind) {
+  Shared& sh = shared();
+  if (blockIdx.x != 0) return;
+  const unsigned long long t = globaltimer_ns();
+  sh.acc[kind] += t - sh.t_last;
+  sh.t_last = t;
+}
+
+// The work items of MARK (it starts, push and pull: which halves) and EVAL.
+template <int V>
+__device__ __forceinline__ void plan_mark(int r, bool push, bool pull) {
+  Shared& sh = shared();
+  const Env& E = sh.E;
+  const LoopState& in = sh.snap;
+  Work& w = sh.work;
+  const unsigned cA = push ? (unsigned)min((long long)in.q[Q_PUSH].countA, E.qb[0].capA) : 0;
+  const unsigned cU = push ? (unsigned)min((long long)in.q[Q_PUSH].countU, E.qb[0].capU) : 0;
+  const unsigned len = pull ? (unsigned)min((long long)in.m_len[r], E.mem_cap) : 0;
+  // units go in up to four pieces while there are warps for them; a short
+  // member list is spread over the warps left
+  w.us = unit_pieces(cU, E.nwarps);
+  w.units = cU << w.us;
+  const unsigned free = E.nwarps > 2 * w.units ? E.nwarps - w.units : E.nwarps / 2;
+  w.ms = share(len, free, 5);
+  if ((free << w.ms) < len) w.ms = V == DC_HB ? 7 : 6;  // as many as pull_members takes at once
+  w.members = w.units + shares(len, w.ms);
+  w.as = batch_share(cA, w.members, E.nwarps);
+  w.total = w.members + shares(cA, w.as);
+  w.sh = grab_share(w.total, E.nwarps);
+}
+__device__ __forceinline__ void plan_eval(int r) {
+  Shared& sh = shared();
+  const Env& E = sh.E;
+  const LoopState& in = sh.snap;
+  Work& w = sh.work;
+  const unsigned cS = (unsigned)min((long long)in.q[Q_SCAN].countU, E.qb[1].capU);
+  const unsigned cA = (unsigned)min((long long)in.q[Q_EVAL + r].countA, E.qb[2].capA);
+  const unsigned cU = (unsigned)min((long long)in.q[Q_EVAL + r].countU, E.qb[2].capU);
+  w.us = unit_pieces(cS, E.nwarps);
+  w.units = cS << w.us;
+  w.members = w.units + cU;
+  w.as = batch_share(cA, w.members, E.nwarps);
+  w.total = w.members + shares(cA, w.as);
+  w.sh = grab_share(w.total, E.nwarps);
+}
+
+// The phase after the one that just ended, and its work (one thread).
+template <int V>
+__device__ __noinline__ void next_phase(long long iter_cap) {
+  Shared& sh = shared();
+  const Env& E = sh.E;
+  const LoopState& in = sh.snap;
+  Step& S = sh.step;
+  const int r = S.r;
+  int ph = S.ph;
+  auto filled = [&](int q) { return in.q[q].countA + in.q[q].countU > 0; };
+  bool next_it = false;
+  switch (ph) {
+    case P_D1: ph = filled(Q_S1) ? P_D2 : P_I1; break;
+    case P_D2: ph = P_D3; break;
+    case P_D3: ph = P_I1; break;
+    case P_I1: ph = filled(Q_S2E) ? P_I2 : P_F0; break;
+    case P_I2: ph = P_I3; break;
+    case P_I3: ph = P_I4; break;
+    case P_I4: ph = P_I5; break;
+    case P_I5: ph = P_F0; break;
+    case P_H1: ph = filled(Q_S1) ? P_H2 : P_F0; break;
+    case P_H2: ph = P_H3; break;
+    case P_H3: ph = P_F0; break;
+    case P_F0: case P_APPEND0:
+      if (ph == P_F0 && V == DC_HI && E.hri_on && in.a_count > 0) {
+        ph = P_APPEND0;
+        break;
+      }
+      lap(0);
+      if (filled(Q_PUSH))
+        next_it = true;
+      else
+        ph = P_END;
+      break;
+    case P_MARK:
+      if (V == DC_HI && S.it == 1) {
+        ph = P_PULL;
+        break;
+      }
+      [[fallthrough]];
+    case P_PULL:
+      lap(1);
+      if (in.ev_rows[r] + in.q[Q_SCAN].countU > 0) {
+        ph = P_EVAL;
+        break;
+      }
+      [[fallthrough]];
+    case P_EVAL: {
+      if (ph == P_EVAL) lap(2);
+      const long long q = next_members(in, r);
+      if (blockIdx.x == 0) sh.frontiers += q;
+      if ((V == DC_HI && q == 0) || (V == DC_HB && in.ev_rows[r] == 0))
+        ph = P_END;  // HB: every mex stands, no colour changes
+      else
+        ph = P_COMMIT;
+      break;
+    }
+    case P_COMMIT: case P_APPEND:
+      if (ph == P_COMMIT && V == DC_HB && in.chg[r] == 0) {
+        lap(3);
+        ph = P_END;
+      } else if (ph == P_COMMIT && V == DC_HI && E.hri_on && in.a_count > 0) {
+        ph = P_APPEND;
+      } else {
+        // the next iteration, with a rebuilt member list
+        next_it = true;
+      }
+      break;
+    case P_REBUILD:
+      ph = P_MARK;
+      lap(3);
+      break;
+    default: break;
+  }
+  if (next_it) {
+    if (S.it > 0) lap(3);
+    if (S.it >= iter_cap) {
+      if (blockIdx.x == 0) atomicOr(&E.st->status, ST_ITER);
+      ph = P_END;
+    } else {
+      ++S.it;
+      S.r = S.rn;
+      S.rn = S.rn == 2 ? 0 : S.rn + 1;
+      ph = S.it > 1 && in.m_rebuild[S.r] != 0u ? P_REBUILD : P_MARK;
+    }
+  }
+  S.ph = ph;
+  S.ps = S.ps == 2 ? 0 : S.ps + 1;
+  if (ph == P_MARK || ph == P_PULL)
+    plan_mark<V>(S.r, ph == P_MARK, ph == P_PULL || V == DC_HB || S.it > 1);
+  else if (ph == P_EVAL)
+    plan_eval(S.r);
 }
 
 // The line phases of the seeding.
@@ -1978,6 +2151,7 @@ __device__ __forceinline__ void setup_env(const RecolorParams& p) {
     E.st = p.st;
     E.ls = &p.st->ls;
     E.nwarps = gridDim.x * kWarps;
+    E.loop_units = min(p.unit_slots, kLoopUnit);
 #pragma unroll 1
     for (int i = 0; i < 3; ++i) E.qb[i] = p.qb[i];
     E.bmA = p.bmA;
@@ -2001,6 +2175,7 @@ __device__ __forceinline__ void setup_env(const RecolorParams& p) {
 #pragma unroll 1
     for (int i = 0; i < 4; ++i) sh.acc[i] = 0;
     sh.frontiers = sh.sorted = 0;
+    sh.step = Step{P_END, 0, 0, 1, 0};
   }
   if (lane_id() == 0) sh.scanned[warp_id()] = sh.idx_cov[warp_id()] = sh.idx_reads[warp_id()] = 0;
   if (lane_id() < 4) sh.cov[warp_id()][lane_id()] = 0;
@@ -2025,6 +2200,7 @@ __global__ void __launch_bounds__(kThreads, 2) recolor_kernel(const __grid_const
   if (threadIdx.x == 0) {
     E.hri_on = V == DC_HI && p.hri.min_live > 0;
     E.hri_split = V == DC_HB && p.hri.min_live > 0;
+    sh.step.ph = V == DC_HI ? P_D1 : P_H1;
     if (p.gid) {
       E.gcount = V == DC_HI ? p.gcnt : nullptr;
       E.gf0 = p.gf0;
@@ -2036,29 +2212,18 @@ __global__ void __launch_bounds__(kThreads, 2) recolor_kernel(const __grid_const
         ld_cg(reinterpret_cast<unsigned*>(&st->ls) + threadIdx.x);
   __syncthreads();
 
-  // Phase timer: CTA 0 thread 0 reads %globaltimer after each barrier and
-  // charges the elapsed time to the phase kind that just ended.
   if (leader) st->t_recolor[0] = sh.t_last = globaltimer_ns();
-  auto lap = [&](int kind) {
-    if (leader) {
-      const unsigned long long t = globaltimer_ns();
-      sh.acc[kind] += t - sh.t_last;
-      sh.t_last = t;
-    }
-  };
   const long long K = p.k_dev ? *p.k_dev : p.k;
   constexpr int rmode = V == DC_HI ? M_MEX_ALL : M_MEX_PRIOR;
 
-  int ps = 0;         // phase sequence for the work-grab ring
-  long long it = 0;
-  int r = 0, rn = 1;  // it % 3, (it + 1) % 3
-  int ph = V == DC_HI ? P_D1 : P_H1;
-
-  while (ph != P_END) {
+  while (true) {
+    const int ph = sh.step.ph, r = sh.step.r, rn = sh.step.rn;
+    const long long it = sh.step.it;
+    if (ph == P_END) break;
     LoopState* ls = &st->ls;
     const LoopState& in = sh.snap;
     int* gprv = nullptr;  // HB, batched: colour changes per graph in the previous iteration
-    if (V == DC_HB && p.gid) {
+    if (V == DC_HB && E.gid) {
       gprv = p.gcnt + (it & 1 ? 0 : (long long)p.ngraphs);
       if (threadIdx.x == 0) {
         E.gchg = p.gcnt + (it & 1 ? (long long)p.ngraphs : 0);
@@ -2068,13 +2233,13 @@ __global__ void __launch_bounds__(kThreads, 2) recolor_kernel(const __grid_const
     }
     // Counter the warps take work items from; the next phase's, last used two
     // phases ago, is cleared.
+    const int ps = sh.step.ps;
     unsigned* ctr = &st->ctl[1].wctr[ps];
-    ps = ps == 2 ? 0 : ps + 1;
-    if (leader) st->ctl[1].wctr[ps] = 0u;
+    if (leader) st->ctl[1].wctr[ps == 2 ? 0 : ps + 1] = 0u;
     // Unit size of the rows pushed for a seeding phase of about `items` work
-    // items, and of the loop's rows.
+    // items.
     auto units_for = [&](unsigned items) { return unit_slots_for(items, E.nwarps, p.unit_slots); };
-    const int loop_units = min(p.unit_slots, kLoopUnit);
+    const int loop_units = E.loop_units;
 
     // ---------------- the phase ----------------
     switch (ph) {
@@ -2108,7 +2273,7 @@ __global__ void __launch_bounds__(kThreads, 2) recolor_kernel(const __grid_const
         // F0 is complete: it becomes the loop's first frontier, and all of
         // it pushes in the first iteration
         phase_frontier0<V>();
-        if (p.gid) {
+        if (E.gid) {
           // a graph whose seeding recoloured nothing never enters the loop
 #pragma unroll 1
           for (long long gg = gtid; gg < p.ngraphs; gg += gthreads) p.gstate[gg] = p.gf0[gg] > 0 ? 1 : 2;
@@ -2130,7 +2295,7 @@ __global__ void __launch_bounds__(kThreads, 2) recolor_kernel(const __grid_const
           ls->a_count = 0;
           ls->m_build = 0;
         }
-        if (V == DC_HB && p.gid && it > 1) {
+        if (V == DC_HB && E.gid && it > 1) {
           // graphs with no colour change in the previous iteration are done
           // (the reference's loop would have ended for them)
           for (long long gg = gtid; gg < p.ngraphs; gg += gthreads)
@@ -2139,12 +2304,11 @@ __global__ void __launch_bounds__(kThreads, 2) recolor_kernel(const __grid_const
               p.giters[gg] = (int)(it - 1);
             }
         }
-        phase_mark<V>(Target{2, (short)(Q_EVAL + r), R_EVAL, loop_units, it == 1}, (int)it, r, ph == P_MARK,
-                      ph == P_PULL || V == DC_HB || it > 1, ctr);
+        phase_mark<V>(Target{2, (short)(Q_EVAL + r), R_EVAL, loop_units, it == 1}, (int)it, r, ctr);
         break;
       case P_EVAL:
         if (leader) ls->q[Q_PUSH] = QCount{0, 0, 0, 0};  // consumed
-        phase_eval<V>(Target{2, (short)(Q_EVAL + r), R_EVAL, loop_units, false}, (int)it, r, ctr, rmode, p.ncolor);
+        phase_eval<V>(Target{2, (short)(Q_EVAL + r), R_EVAL, loop_units, false}, (int)it, r, ctr, rmode, E.ncolor);
         break;
       case P_COMMIT: {
         const long long tail = (long long)in.m_tail;
@@ -2161,7 +2325,7 @@ __global__ void __launch_bounds__(kThreads, 2) recolor_kernel(const __grid_const
           ls->m_rebuild[rn] = rebuild ? 1u : 0u;
           if (rebuild) sh.sorted = q;
         }
-        if (p.gid) {
+        if (E.gid) {
 #pragma unroll 1
           for (long long gg = gtid; gg < p.ngraphs; gg += gthreads) {
             if (V == DC_HB) {
@@ -2184,89 +2348,11 @@ __global__ void __launch_bounds__(kThreads, 2) recolor_kernel(const __grid_const
         break;
     }
 
-    // ---------------- its barrier ----------------
-    if (!sync_grid(st, p.bar_timeout_ns)) return;
-
-    // ---------------- the next phase ----------------
-    auto filled = [&](int q) { return in.q[q].countA + in.q[q].countU > 0; };
-    bool next_it = false;
-    switch (ph) {
-      case P_D1: ph = filled(Q_S1) ? P_D2 : P_I1; break;
-      case P_D2: ph = P_D3; break;
-      case P_D3: ph = P_I1; break;
-      case P_I1: ph = filled(Q_S2E) ? P_I2 : P_F0; break;
-      case P_I2: ph = P_I3; break;
-      case P_I3: ph = P_I4; break;
-      case P_I4: ph = P_I5; break;
-      case P_I5: ph = P_F0; break;
-      case P_H1: ph = filled(Q_S1) ? P_H2 : P_F0; break;
-      case P_H2: ph = P_H3; break;
-      case P_H3: ph = P_F0; break;
-      case P_F0: case P_APPEND0:
-        if (ph == P_F0 && V == DC_HI && E.hri_on && in.a_count > 0) {
-          ph = P_APPEND0;
-          break;
-        }
-        lap(0);
-        if (filled(Q_PUSH))
-          next_it = true;
-        else
-          ph = P_END;
-        break;
-      case P_MARK:
-        if (V == DC_HI && it == 1) {
-          ph = P_PULL;
-          break;
-        }
-        [[fallthrough]];
-      case P_PULL:
-        lap(1);
-        if (in.ev_rows[r] + in.q[Q_SCAN].countU > 0) {
-          ph = P_EVAL;
-          break;
-        }
-        [[fallthrough]];
-      case P_EVAL: {
-        if (ph == P_EVAL) lap(2);
-        const long long q = next_members(in, r);
-        if (leader) sh.frontiers += q;
-        if ((V == DC_HI && q == 0) || (V == DC_HB && in.ev_rows[r] == 0))
-          ph = P_END;  // HB: every mex stands, no colour changes
-        else
-          ph = P_COMMIT;
-        break;
-      }
-      case P_COMMIT: case P_APPEND:
-        if (ph == P_COMMIT && V == DC_HB && in.chg[r] == 0) {
-          lap(3);
-          ph = P_END;
-        } else if (ph == P_COMMIT && V == DC_HI && E.hri_on && in.a_count > 0) {
-          ph = P_APPEND;
-        } else {
-          // the next iteration, with a rebuilt member list
-          next_it = true;
-        }
-        break;
-      case P_REBUILD:
-        ph = P_MARK;
-        lap(3);
-        break;
-      default: break;
-    }
-    if (next_it) {
-      if (it > 0) lap(3);
-      if (it >= p.iter_cap) {
-        if (leader) atomicOr(&st->status, ST_ITER);
-        ph = P_END;
-      } else {
-        ++it;
-        r = rn;
-        rn = rn == 2 ? 0 : rn + 1;
-        ph = it > 1 && in.m_rebuild[r] != 0u ? P_REBUILD : P_MARK;
-      }
-    }
+    // ---------------- its barrier, and the next phase ----------------
+    if (!sync_grid(st, p.bar_timeout_ns, [&] { next_phase<V>(p.iter_cap); })) return;
   }
 
+  const long long it = sh.step.it;
   // ---------------- the end ----------------
   // the membership bits and the flags they stand for, and the clean bits
   {
