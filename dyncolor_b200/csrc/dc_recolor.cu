@@ -2416,96 +2416,189 @@ __global__ void __launch_bounds__(kThreads, 2) recolor_kernel(const __grid_const
 // comparison); with g.prop all zero it is the vertex-id order.
 //   P   pred[v] = neighbours before v         (all vertices, in units)
 //   F   frontier F0 = vertices with pred 0
-//   round (until the frontier is empty):
-//     R  mex over the neighbours before v      -> ncolor
-//     D  commit the colour; every neighbour after v loses one pred, and the
-//        ones that reach 0 form the next frontier
+//   round (until the frontier is empty): one walk of each frontier row takes
+//     the mex over the neighbours before v, which is v's colour, and one pred
+//     from every neighbour after v; the ones that reach 0 form the next
+//     frontier
+// The vertices of a round are independent (an edge between two of them would
+// leave the later one a pred), so a round reads no colour that it writes, and
+// the next round starts behind its barrier.  A round of a few dozen vertices
+// is bound by its chain of dependent trips to L2 and its barrier.  R-MAT scale
+// 18, 3.8 M edges, LDF, 859 rounds: 18.0 ms; with a phase for the mex and one
+// for the release, units of 4096 slots walked 32 at a time and a lane per
+// class-A row it took 49.
 // ---------------------------------------------------------------------
 namespace {
 
-// P over one unit (or a class-A batch of 32 rows): counts the neighbours of
-// each row that come before it.
-__device__ void pred_unit(const GraphDev& g, int4 un, int* pred) {
+// P over one unit, and a class-A batch: counts the neighbours of each row
+// that come before it.
+__device__ __noinline__ void pred_unit(int4 un, int* pred) {
+  const GraphDev& g = env().g;
   const int v = un.x;
-  const int L = g.len[v];
-  const long long o = g.off[v];
-  const int us = unit_span(L, un.w);
-  const int s_lo = un.y * us, s_hi = min(L, s_lo + us);
-  const int pv = g.prop[v];
-  int cnt = 0;
-#pragma unroll 1
-  for (int s0 = s_lo; s0 < s_hi; s0 += 32) {
-    const int sidx = s0 + lane_id();
-    const int u = sidx < s_hi ? g.adj[o + sidx] : -1;
-    if (u >= 0 && is_prior(g.prop[u], u, pv, v)) ++cnt;
-  }
-  cnt = __reduce_add_sync(0xffffffffu, cnt);
-  if (lane_id() == 0 && cnt) atomicAdd(&pred[v], cnt);
-}
-
-__device__ void pred_batchA(const GraphDev& g, const int* items, unsigned cA, unsigned b, int* pred) {
-  const unsigned idx = b * 32 + lane_id();
-  if (idx >= cA) return;
-  const int v = items[idx];
-  const int L = g.len[v];
-  const long long o = g.off[v];
-  const int pv = g.prop[v];
-  int cnt = 0;
-#pragma unroll 1
-  for (int s = 0; s < L; ++s) {
-    const int u = g.adj[o + s];
-    if (u >= 0 && is_prior(g.prop[u], u, pv, v)) ++cnt;
-  }
-  if (cnt) atomicAdd(&pred[v], cnt);
-}
-
-// Commits v's colour (its first unit) into the colour word and the packed
-// word.
-__device__ __forceinline__ int commit_init(const Env& E, int v) {
-  const int c = E.ncolor[v];
-  E.g.color[v] = c;
-  *flag_word<DC_HB>(E, v) = (unsigned)c;
-  return c;
-}
-
-// D over one unit: every neighbour after v loses one pred; those reaching 0
-// are ready.
-__device__ __noinline__ void release_unit(Target T, int4 un, int* pred, int& cmax) {
-  const Env& E = env();
-  const GraphDev& g = E.g;
-  const int v = un.x;
-  if (un.y == 0 && lane_id() == 0) cmax = max(cmax, commit_init(E, v));
   const int L = g.len[v];
   const int* adj = g.adj + g.off[v];
   const int us = unit_span(L, un.w);
   const int s_lo = un.y * us, s_hi = min(L, s_lo + us);
   const int pv = g.prop[v];
+  int cnt = 0;
 #pragma unroll 1
-  for (int s = s_lo + lane_id(); s < s_hi; s += 32) {
-    const int u = adj[s];
-    if (u >= 0 && is_prior(pv, v, g.prop[u], u) && atomicSub(&pred[u], 1) == 1) stage(T, u);
+  for (int s0 = s_lo + lane_id(); s0 < s_hi; s0 += 128) {
+    int uu[4], pp[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) uu[j] = s0 + j * 32 < s_hi ? adj[s0 + j * 32] : -1;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) pp[j] = uu[j] >= 0 ? g.prop[uu[j]] : 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) cnt += uu[j] >= 0 && is_prior(pp[j], uu[j], pv, v);
   }
+  __syncwarp();
+  cnt = __reduce_add_sync(0xffffffffu, cnt);
+  if (lane_id() == 0 && cnt) atomicAdd(&pred[v], cnt);
+}
+
+__device__ __noinline__ void pred_batchA(const int* items, unsigned cA, unsigned idx, int* pred) {
+  Shared& sh = shared();
+  const GraphDev& g = sh.E.g;
+  const bool valid = idx < cA;
+  const int v = valid ? items[idx] : 0;
+  Rows& R = sh.rows[warp_id()];
+  R.a[lane_id()] = v;
+  R.b[lane_id()] = valid ? g.prop[v] : 0;
+  R.c[lane_id()] = 0;
+  const int T = number_rows(R, g.adj + (valid ? g.off[v] : 0), valid ? g.len[v] : 0);
+#pragma unroll 1
+  for (int s0 = lane_id(); s0 < T; s0 += 128) {
+    int jj[4], uu[4], pp[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int s = s0 + r * 32;
+      jj[r] = row_of(R, s);
+      uu[r] = s < T ? R.at[jj[r]][s - R.excl[jj[r]]] : -1;
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r) pp[r] = uu[r] >= 0 ? g.prop[uu[r]] : 0;
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+      if (uu[r] >= 0 && is_prior(pp[r], uu[r], R.b[jj[r]], R.a[jj[r]])) atomicAdd(&R.c[jj[r]], 1);
+  }
+  __syncwarp();
+  if (valid) pred[v] = R.c[lane_id()];
   __syncwarp();
 }
 
-__device__ __noinline__ void release_batchA(Target T, const int* items, unsigned cA, unsigned b, int* pred,
-                                            int& cmax) {
-  const Env& E = env();
-  const GraphDev& g = E.g;
-  const unsigned idx = b * 32 + lane_id();
-  if (idx < cA) {
-    const int v = items[idx];
-    cmax = max(cmax, commit_init(E, v));
-    const int L = g.len[v];
-    const int* adj = g.adj + g.off[v];
-    const int pv = g.prop[v];
+// v's colour into the colour word and the packed word.
+__device__ __forceinline__ void commit_init(const Env& E, int v, int c) {
+  E.g.color[v] = c;
+  *flag_word<DC_HB>(E, v) = (unsigned)c;
+}
+
+// U neighbours per lane: those after their row lose one pred; the ones that
+// reach 0 are ready.
+template <int U>
+__device__ __forceinline__ void release(Target T, const int* uu, unsigned after, int* pred) {
+  int left[U];
+#pragma unroll
+  for (int j = 0; j < U; ++j) left[j] = (after >> j) & 1u ? atomicSub(&pred[uu[j]], 1) : 0;
+#pragma unroll
+  for (int j = 0; j < U; ++j)
+    if (left[j] == 1) stage(T, uu[j]);
+}
+
+// A round's walk of one unit of a row.  Returns the row's colour where this
+// unit finished it, else -1.
+__device__ __noinline__ int color_unit(Target T, int4 un, const unsigned* gmask, int* pred) {
+  Shared& sh = shared();
+  const Env& E = sh.E;
+  const int v = un.x;
+  const int L = E.g.len[v];
+  const int* adj = E.g.adj + E.g.off[v];
+  const int us = unit_span(L, un.w);
+  const int s_lo = un.y * us, s_hi = min(L, s_lo + us);
+  const int limit = min(L, kMaskBits), nw = mask_words(L, M_MEX_PRIOR);
+  const int pv = E.g.prop[v];
+  unsigned* sm = sh.mask[warp_id()];
 #pragma unroll 1
-    for (int s = 0; s < L; ++s) {
-      const int u = adj[s];
-      if (u >= 0 && is_prior(pv, v, g.prop[u], u) && atomicSub(&pred[u], 1) == 1) stage(T, u);
+  for (int k = lane_id(); k < nw; k += 32) sm[k] = 0;
+  __syncwarp();
+  unsigned long long lm = 0;  // colours < 64 seen by this lane
+  // eight slots per lane per round: a round is a chain of three dependent
+  // trips to L2, whatever its width
+  constexpr int U = 8;
+#pragma unroll 1
+  for (int r0 = s_lo + lane_id(); r0 < s_hi; r0 += 32 * U) {
+    int uu[U];
+    unsigned long long xx[U];
+    unsigned after = 0;
+#pragma unroll
+    for (int j = 0; j < U; ++j) uu[j] = r0 + j * 32 < s_hi ? adj[r0 + j * 32] : -1;
+#pragma unroll
+    for (int j = 0; j < U; ++j) xx[j] = uu[j] >= 0 ? E.cp[uu[j]] : 0ull;
+#pragma unroll
+    for (int j = 0; j < U; ++j) {
+      if (uu[j] < 0) continue;
+      if (!is_prior((int)(xx[j] >> 32), uu[j], pv, v)) {
+        after |= 1u << j;
+        continue;
+      }
+      const int c = (int)(unsigned)xx[j];
+      if (c < 64)
+        lm |= 1ull << c;
+      else if (c < limit)
+        atomicOr(&sm[c >> 5], 1u << (c & 31));
     }
+    release<U>(T, uu, after, pred);
   }
   __syncwarp();
+  fold_low(sm, lm);
+  if (un.w > 1 && !merge_masks(const_cast<unsigned*>(gmask) + un.z, sm, nw, un.w)) return -1;
+  int r = first_zero(sm, nw);
+  __syncwarp();
+  if (r < 0) r = slow_mex(v, M_MEX_PRIOR, kMaskBits);
+  if (lane_id() == 0) commit_init(E, v, r);
+  __syncwarp();
+  return r;
+}
+
+// The same of a class-A batch.  Returns each lane's row's colour (-1: none).
+__device__ __noinline__ int color_batchA(Target T, const int* items, unsigned cA, unsigned idx, int* pred) {
+  Shared& sh = shared();
+  const Env& E = sh.E;
+  const bool valid = idx < cA;
+  const int v = valid ? items[idx] : 0;
+  Rows& R = sh.rows[warp_id()];
+  unsigned long long* m64 = reinterpret_cast<unsigned long long*>(sh.mask[warp_id()]);
+  m64[lane_id()] = 0ull;
+  R.a[lane_id()] = v;
+  R.b[lane_id()] = valid ? E.g.prop[v] : 0;
+  const int S = number_rows(R, E.g.adj + (valid ? E.g.off[v] : 0), valid ? E.g.len[v] : 0);
+#pragma unroll 1
+  for (int s0 = lane_id(); s0 < S; s0 += 128) {
+    int jj[4], uu[4];
+    unsigned long long xx[4];
+    unsigned after = 0;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int s = s0 + r * 32;
+      jj[r] = row_of(R, s);
+      uu[r] = s < S ? R.at[jj[r]][s - R.excl[jj[r]]] : -1;
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r) xx[r] = uu[r] >= 0 ? E.cp[uu[r]] : 0ull;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const bool before = uu[r] >= 0 && is_prior((int)(xx[r] >> 32), uu[r], R.b[jj[r]], R.a[jj[r]]);
+      if (uu[r] >= 0 && !before) after |= 1u << r;
+      const int c = (int)(unsigned)xx[r];
+      // a class-A row has at most 32 neighbours: its colour is below 64
+      if (before && c < 64) atomicOr(reinterpret_cast<unsigned*>(&m64[jj[r]]) + (c >> 5), 1u << (c & 31));
+    }
+    release<4>(T, uu, after, pred);
+  }
+  __syncwarp();
+  const int c = valid ? __ffsll((long long)~m64[lane_id()]) - 1 : -1;
+  if (valid) commit_init(E, v, c);
+  __syncwarp();
+  return c;
 }
 
 }  // namespace
@@ -2520,7 +2613,7 @@ __global__ void __launch_bounds__(kThreads, 2) init_color_kernel(const __grid_co
   int* pred = p.pred;
   const unsigned gwarp = team_warp(), nwarps = E.nwarps;
   const bool leader = blockIdx.x == 0 && threadIdx.x == 0;
-  const int CH = p.unit_slots;
+  const int CH = E.loop_units;
   int ps = 0;
   auto ctr = [&]() -> unsigned* {
     unsigned* c = &st->ctl[1].wctr[ps];
@@ -2545,14 +2638,15 @@ __global__ void __launch_bounds__(kThreads, 2) init_color_kernel(const __grid_co
     const QCount& qc = sh.snap.q[Q_S1];
     const unsigned cA = (unsigned)min((long long)qc.countA, qb.capA);
     const unsigned cU = (unsigned)min((long long)qc.countU, qb.capU);
-    Grabber gb(ctr(), cU + (cA + 31) / 32, gwarp, nwarps);
+    const int as = batch_share(cA, cU, nwarps);
+    Grabber gb(ctr(), cU + shares(cA, as), gwarp, nwarps);
     unsigned i;
 #pragma unroll 1
     while (gb.next(i)) {
       if (i < cU)
-        pred_unit(g, qb.units[i], pred);
+        pred_unit(qb.units[i], pred);
       else
-        pred_batchA(g, qb.itemsA, cA, i - cU, pred);
+        pred_batchA(qb.itemsA, cA, batch_item(i - cU, as), pred);
     }
   }
   if (!sync_grid(st, p.bar_timeout_ns)) return;
@@ -2576,27 +2670,19 @@ __global__ void __launch_bounds__(kThreads, 2) init_color_kernel(const __grid_co
     const int ns = fs == 2 ? 0 : fs + 1;
     const int nb = fb ^ 1;
     if (leader) st->ls.q[ns == 2 ? 0 : ns + 1] = QCount{0, 0, 0, 0};
-    // R: the mex over the neighbours before each frontier vertex
-    phase_reduce<DC_HB>(fb, fs, ctr(), M_MEX_PRIOR, true, p.ncolor);
-    if (!sync_grid(st, p.bar_timeout_ns)) return;
-    // D
-    {
-      const QueueBufs& fq = p.qb[fb];
-      const QCount& fc = sh.snap.q[fs];
-      const unsigned cA = (unsigned)min((long long)fc.countA, fq.capA);
-      const unsigned cU = (unsigned)min((long long)fc.countU, fq.capU);
-      const Target T = {(short)nb, (short)ns, R_MEX, CH};
-      Grabber gb(ctr(), cU + (cA + 31) / 32, gwarp, nwarps);
-      unsigned i;
+    const QueueBufs& fq = p.qb[fb];
+    const QCount& fc = sh.snap.q[fs];
+    const unsigned cA = (unsigned)min((long long)fc.countA, fq.capA);
+    const unsigned cU = (unsigned)min((long long)fc.countU, fq.capU);
+    const Target T = {(short)nb, (short)ns, R_MEX, CH};
+    const int as = batch_share(cA, cU, nwarps);
+    Grabber gb(ctr(), cU + shares(cA, as), gwarp, nwarps);
+    unsigned i;
 #pragma unroll 1
-      while (gb.next(i)) {
-        if (i < cU)
-          release_unit(T, fq.units[i], pred, cmax);
-        else
-          release_batchA(T, fq.itemsA, cA, i - cU, pred, cmax);
-      }
-      finish_push(T);
-    }
+    while (gb.next(i))
+      cmax = max(cmax, i < cU ? color_unit(T, fq.units[i], fq.gmask, pred)
+                              : color_batchA(T, fq.itemsA, cA, batch_item(i - cU, as), pred));
+    finish_push(T);
     if (!sync_grid(st, p.bar_timeout_ns)) return;
     fs = ns;
     fb = nb;

@@ -143,3 +143,19 @@ def test_every_row_just_past_the_short_search(variant, ov, degree):
         assert (sg.iterations, sg.seed_targets, sg.frontier_total) == (
             so.iterations, so.seed_targets, so.frontier_total)
     ctx.close()
+
+
+@pytest.mark.parametrize("order", [dc.ORDER_ID, dc.ORDER_LDF])
+@pytest.mark.parametrize("kw", [{}, dict(unit_slots=128), dict(grid_ctas=1)])
+def test_initial_colouring_of_rows_at_the_edges_of_its_units(order, kw):
+    n, a, b = _hubs(3000, seed=5)
+    deg = np.bincount(np.concatenate([a, b]), minlength=n)
+    seq = np.arange(n) if order == dc.ORDER_ID else np.lexsort((np.arange(n), -deg))
+    ctx = dc.Context(variant=dc.HB, **kw)
+    ctx.load_edges(n, a, b)
+    g = oracle_graph(n, a, b, np.zeros(n, np.int32))
+    for _ in range(2):
+        ctx.init_colors(order)
+        g.greedy_in_order(seq.astype(np.int32))
+        assert np.array_equal(ctx.colors(), g.colors())
+    ctx.close()
