@@ -414,10 +414,12 @@ __device__ __forceinline__ void write_member(const Env& E, unsigned at, int u) {
 
 // Pushes u (any subset of the warp calls): vertices collect in the CTA's
 // buffer, which finish_push moves on at the end of the phase with one atomic
-// per counter; what does not fit goes to its queue at once.
+// per counter; what does not fit goes to its queue at once.  (Lanes take their
+// places one by one: finding the ones that could share an atomic cost 1 - 5 %
+// of a batch, 7.7 -> 7.3 ms for 96 graphs.)
 __device__ __noinline__ void stage(Target T, int u) {
   Shared& sh = shared();
-  const unsigned at = take_one(&sh.ccnt);
+  const unsigned at = atomicAdd(&sh.ccnt, 1u);
   if (at < kCtaBuf) {
     sh.cbuf[at] = u;
     return;
@@ -434,7 +436,7 @@ __device__ __noinline__ void stage(Target T, int u) {
 // u enters the frontier: the same for the end of the member list.
 __device__ __noinline__ void stage_member(int u) {
   Shared& sh = shared();
-  const unsigned at = take_one(&sh.mcnt);
+  const unsigned at = atomicAdd(&sh.mcnt, 1u);
   if (at < kMemBuf)
     sh.mbuf[at] = u;
   else
