@@ -402,7 +402,6 @@ constexpr long long kOneCtaPerSmLines = 32768;
 int struct_grid(const dc_ctx* ctx, long long k) {
   return k <= kOneCtaPerSmLines ? std::min(ctx->grid_struct, ctx->sms) : ctx->grid_struct;
 }
-
 // Enqueues one attempt of a batch (or load) on the context's stream, ending
 // with the copy of the device state into pinned host memory.  k_dev, when
 // set, makes the kernels read the line count from device memory, so a
@@ -416,7 +415,9 @@ dc_status enqueue_batch(dc_ctx* ctx, const dc_change* d_ch, const int* la, const
   StructParams sp = struct_params(ctx, d_ch, la, lb, k);
   sp.k_dev = k_dev;
   // (a captured sequence serves every batch that the scratch can hold)
-  DC_CK(launch_struct(sp, struct_grid(ctx, k_dev ? ctx->kcap : k), ctx->stream));
+  const long long lines = k_dev ? ctx->kcap : k;
+  sp.small_keys = k_dev || 2 * k <= kSmallKeys ? kSmallKeys : 0;
+  DC_CK(launch_struct(sp, struct_grid(ctx, lines), ctx->stream));
   if (events) DC_CK(cudaEventRecord(ctx->evm, ctx->stream));
   if (recolor) {
     if (ctx->ngraphs > 0) {

@@ -35,6 +35,7 @@ constexpr int kNumQueues = 8;       // logical queue counter slots
 constexpr long long kMemSlack = 4096;     // member-list entries the loop may add beyond half the live ones before a rebuild
 constexpr int kUnitSlotsDefault = 4096;  // adjacency slots per warp work unit
 constexpr int kLoopUnit = 512;           // slots per work unit of the recolour loop's rows, at most
+constexpr int kSmallKeys = 4096;         // keys of a small batch's shared-memory sort (two buffers)
 constexpr int kScanBatch = 32;           // witness searches up to this length are taken 32 rows at a time
 constexpr int kScanWords = 4;            // mask region of a longer one that goes on in units
 constexpr int kPushWords = 12;           // mask region of a pushing indexed row (the last five fields of its plan)
@@ -170,6 +171,7 @@ struct StructParams {
   long long cap_rel;
   const int* gid;        // batched mode: vertex -> graph; lines must stay inside a graph
   unsigned long long bar_timeout_ns;  // limit of every grid-barrier wait
+  int small_keys;  // keys that the two buffers in dynamic shared memory hold
   DevState* st;
 };
 

@@ -59,6 +59,20 @@ __device__ __forceinline__ int warp_atomic_add32(int* ctr, int val) {
   return base + incl - val;
 }
 
+// Lanes of `act` (all call) with this lane's 8-bit digit: a ballot per bit
+// (__match_any_sync slows with every distinct value; a batch of 5000 lines
+// sorted by one CTA: 185 us with it, 168 with ballots).
+__device__ __forceinline__ unsigned same_digit(unsigned act, unsigned d) {
+  unsigned m = act;
+#pragma unroll
+  for (int b = 0; b < 8; ++b) {
+    const bool on = (d >> b) & 1u;
+    const unsigned bal = __ballot_sync(act, on);
+    m &= on ? bal : ~bal;
+  }
+  return m;
+}
+
 // The grid barrier of the structural launch; `target` is per-CTA state
 // starting at 0.  All threads call; false once a wait has run out.
 __device__ __noinline__ bool grid_sync(DevState* st, unsigned& target, unsigned long long timeout_ns) {
@@ -69,124 +83,170 @@ __device__ __noinline__ bool grid_sync(DevState* st, unsigned& target, unsigned 
   return s_ok != 0;
 }
 
-// Batches of up to this many keys (two per line) are sorted, netted and cut
-// into row units by CTA 0 alone, in shared memory, while the other CTAs wait
-// at one barrier.  Such a batch is bound by barriers, not by its data: the
-// general path has three per sort pass and six more before the row scans, 27
-// in all at 20 lines.  20 lines on 1000 vertices: 74 us before, 34 now;
-// 101 lines on 3001: 96 -> 49.  The line lies where the keys fill the shared
-// memory that the scatter has anyway; 2048 lines still gain (see the bitonic
-// sort: 66 steps of 2 us at most).
-constexpr int kSmallKeys = 4096;
+// Batches whose keys (two per line) fit the launch's dynamic shared memory
+// (StructParams::small_keys) are sorted, netted and cut into row units by CTA 0
+// alone, while the other CTAs wait at one barrier.  Such a batch is bound by
+// barriers, not by its data: the general path has three per sort pass and six
+// more before the row scans, 27 in all at 20 lines on 1000 vertices.  Whole
+// launch, general path -> this: 20 lines on 1000 vertices 74 -> 34 us, 101 on
+// 3001 96 -> 50, 1000 on 1M 105 -> 67, 2000 111 -> 97; 3000 115 -> 127, so the
+// line is at 2048 lines.
+// Up to kTailKeys keys CTA 0 also decides the capacities and ends the batch
+// alone (500 lines: 54 us); more entries are faster with every CTA and three
+// more barriers (1000 lines: 67 us, 86 alone).
+constexpr int kTailKeys = 1024;
 // Relocation copies a small batch leaves to CTA 0 (units of kStructChunk).
 constexpr int kSmallRel = 64;
 
-// Bitonic sort of n keys (a power of two) in shared memory by one CTA.
-__device__ __noinline__ void sort_shared(unsigned long long* k, int n) {
+// LSD radix sort of n keys of `bits` bits in shared memory by one CTA: 8 bits
+// a pass, each warp its own segment of the keys and its own digit counts
+// (wc).  Returns where the result is, `a` or `b`.
+__device__ __noinline__ unsigned long long* sort_shared(unsigned long long* a, unsigned long long* b, int n, int bits,
+                                                        int (*wc)[256], int* sw) {
+  const int tid = threadIdx.x, w = warp_id();
+  const int seg = (n + kThreads - 1) / kThreads * 32;
+  const int lo = w * seg, hi = min(n, lo + seg);
 #pragma unroll 1
-  for (int size = 2; size <= n; size <<= 1)
+  for (int shift = 0; shift < bits; shift += 8) {
+    for (int i = tid; i < kWarps * 256; i += kThreads) (&wc[0][0])[i] = 0;
+    __syncthreads();
 #pragma unroll 1
-    for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      __syncthreads();
-#pragma unroll 1
-      for (int i = threadIdx.x; i < n / 2; i += kThreads) {
-        const int a = 2 * i - (i & (stride - 1)), b = a + stride;
-        const unsigned long long x = k[a], y = k[b];
-        if ((x > y) == ((a & size) == 0)) {
-          k[a] = y;
-          k[b] = x;
-        }
+    for (int i = lo + lane_id(); i < hi; i += 32) atomicAdd(&wc[w][(unsigned)(a[i] >> shift) & 255u], 1);
+    __syncthreads();
+    // digit starts, then each warp's start within its digits
+    int c = 0;
+    if (tid < 256)
+#pragma unroll
+      for (int k = 0; k < kWarps; ++k) c += wc[k][tid];
+    int tot;
+    int at = block_excl_scan(c, sw, &tot);
+    if (tid < 256)
+#pragma unroll
+      for (int k = 0; k < kWarps; ++k) {
+        const int x = wc[k][tid];
+        wc[k][tid] = at;
+        at += x;
       }
+    __syncthreads();
+#pragma unroll 1
+    for (int i0 = lo; i0 < hi; i0 += 32) {
+      const int i = i0 + lane_id();
+      const bool on = i < hi;
+      const unsigned act = __ballot_sync(0xffffffffu, on);
+      if (on) {
+        const unsigned long long x = a[i];
+        const unsigned d = (unsigned)(x >> shift) & 255u;
+        const unsigned peers = same_digit(act, d);
+        const int to = wc[w][d];
+        __syncwarp(act);
+        if (lane_id() == __ffs(peers) - 1) wc[w][d] = to + __popc(peers);
+        b[to + __popc(peers & lanemask_lt())] = x;
+      }
+      __syncwarp();
     }
-  __syncthreads();
+    __syncthreads();
+    unsigned long long* t = a;
+    a = b;
+    b = t;
+  }
+  return a;
 }
 
 // S0 - S3a of a small batch (see the file comment), by one CTA: keys into
-// `k` (kSmallKeys entries), sorted; netted entries, touched rows and the
+// `k` (twice p.small_keys entries), sorted; netted entries, touched rows and the
 // row-scan units.  False: an invalid line or too many units (status set).
-__device__ __noinline__ bool small_front(const StructParams& p, unsigned long long* k, int K, int* sw, int* flag) {
+__device__ __noinline__ bool small_front(const StructParams& p, unsigned long long* k, int K, int (*wc)[256],
+                                         int* sw, int* flag) {
   DevState* st = p.st;
   const GraphDev& g = p.g;
   const int B = g.key_bits, tid = threadIdx.x;
   const unsigned long long SENT = (1ull << (2 * B + 1)) - 1ull;
-  int P = 2;
-  while (P < 2 * K) P <<= 1;
-  if (tid == 0) flag[0] = flag[1] = 0;
+  if (tid == 0) flag[0] = flag[1] = flag[2] = 0;
   __syncthreads();
-  for (int i = tid; i < P / 2; i += kThreads) {
+  int nv = 0;
+#pragma unroll 4
+  for (int i = tid; i < K; i += kThreads) {
+    int a, b, op = 1;
+    if (p.ch) {
+      const dc_change c = p.ch[i];
+      a = c.node1;
+      b = c.node2;
+      op = c.inst;
+    } else {
+      a = p.la[i];
+      b = p.lb[i];
+    }
     unsigned long long k0 = SENT, k1 = SENT;
-    if (i < K) {
-      int a, b, op = 1;
-      if (p.ch) {
-        const dc_change c = p.ch[i];
-        a = c.node1;
-        b = c.node2;
-        op = c.inst;
+    if (op == 0 || op == 1) {
+      if (a < 0 || a >= g.n || b < 0 || b >= g.n || a == b || (p.gid && p.gid[a] != p.gid[b])) {
+        flag[0] = 1;
       } else {
-        a = p.la[i];
-        b = p.lb[i];
-      }
-      if (op == 0 || op == 1) {
-        if (a < 0 || a >= g.n || b < 0 || b >= g.n || a == b || (p.gid && p.gid[a] != p.gid[b])) {
-          flag[0] = 1;
-        } else {
-          k0 = make_key(a, b, op, B);
-          k1 = make_key(b, a, op, B);
-          atomicAdd(&flag[1], 2);
-        }
+        k0 = make_key(a, b, op, B);
+        k1 = make_key(b, a, op, B);
+        nv += 2;
       }
     }
     k[2 * i] = k0;
     k[2 * i + 1] = k1;
   }
-  sort_shared(k, P);
+  nv = __reduce_add_sync(0xffffffffu, nv);
+  if (lane_id() == 0) atomicAdd(&flag[1], nv);
+  __syncthreads();
   if (flag[0]) {
     if (tid == 0) atomicOr(&st->status, ST_INVAL);
     return false;
   }
-  // netted entries (first of each (row, nbr) group: a delete sorts first) and
-  // touched rows
   const int NV = flag[1];
-  int nn = 0, nt = 0;
+  k = sort_shared(k, k + p.small_keys, 2 * K, 2 * B + 1, wc, sw);
+  // netted entries (first of each (row, nbr) group: a delete sorts first) and
+  // touched rows; each thread takes consecutive keys, so one scan serves all
+  const int per = (NV + kThreads - 1) / kThreads;
+  const int i0 = min(NV, tid * per), i1 = min(NV, i0 + per);
+  const unsigned long long before = i0 > 0 && i0 < NV ? k[i0 - 1] : ~0ull;
+  int nf = 0, nr = 0;
+  unsigned long long y = before;
 #pragma unroll 1
-  for (int t0 = 0; t0 < NV; t0 += kThreads) {
-    const int i = t0 + tid;
-    const unsigned long long x = i < NV ? k[i] : 0ull, y = i > 0 && i < NV ? k[i - 1] : ~0ull;
-    const int f = i < NV && (i == 0 || (x >> 1) != (y >> 1));
-    const int fr = i < NV && (i == 0 || key_row(x, B) != key_row(y, B));
-    int tot;
-    const int ex = block_excl_scan(f | (fr << 16), sw, &tot);
-    if (f) {
-      const int j = nn + (ex & 0xffff), t = nt + (ex >> 16) + fr - 1;
-      p.net[j] = x;
-      p.present[j] = 0;
-      p.tof[j] = t;
-      if (fr) {
+  for (int i = i0; i < i1; ++i) {
+    const unsigned long long x = k[i];
+    nf += i == 0 || (x >> 1) != (y >> 1);
+    nr += i == 0 || key_row(x, B) != key_row(y, B);
+    y = x;
+  }
+  int tot;
+  const int ex = block_excl_scan(nf | (nr << 16), sw, &tot);
+  int j = ex & 0xffff, t = (ex >> 16) - 1;
+  y = before;
+#pragma unroll 1
+  for (int i = i0; i < i1; ++i) {
+    const unsigned long long x = k[i];
+    if (i == 0 || (x >> 1) != (y >> 1)) {
+      if (i == 0 || key_row(x, B) != key_row(y, B)) {
+        ++t;
         p.tbeg[t] = j;
         p.trow[t] = key_row(x, B);
       }
+      p.net[j] = x;
+      p.present[j] = 0;
+      p.tof[j] = t;
+      ++j;
     }
-    nn += tot & 0xffff;
-    nt += tot >> 16;
+    y = x;
   }
+  const int nn = tot & 0xffff, nt = tot >> 16;
   __syncthreads();  // trow is read below by other threads
-  long long units = 0;
-#pragma unroll 1
-  for (int t0 = 0; t0 < nt; t0 += kThreads) {
-    const int t = t0 + tid;
-    int c = 0;
-    if (t < nt) {
-      c = (g.len[p.trow[t]] + kStructChunk - 1) / kStructChunk;
-      p.rowdel[t] = 0;
-      p.tins[t] = 0;
-      p.cursor[t] = 0;
-    }
-    int tot;
-    const int ex = block_excl_scan(c, sw, &tot);
-    if (units + ex + c <= p.cap_units)
-      for (int q = 0; q < c; ++q) p.units[units + ex + q] = make_int2(t, q);
-    units += tot;
+  // (in any order: S3b takes the units from a counter)
+#pragma unroll 4
+  for (int q = tid; q < nt; q += kThreads) {
+    const int c = (g.len[p.trow[q]] + kStructChunk - 1) / kStructChunk;
+    p.rowdel[q] = 0;
+    p.tins[q] = 0;
+    p.cursor[q] = 0;
+    const int at = c > 0 ? atomicAdd(&flag[2], c) : 0;
+    for (int z = 0; z < c; ++z)
+      if (at + z < p.cap_units) p.units[at + z] = make_int2(q, z);
   }
+  __syncthreads();
+  const long long units = flag[2];
   if (tid == 0) {
     st->nvalid = (unsigned long long)(NV / 2);
     st->nnet = (unsigned long long)nn;
@@ -204,13 +264,12 @@ __global__ void __launch_bounds__(kThreads) struct_kernel(StructParams p) {
   __shared__ unsigned s_hist[256];
   __shared__ unsigned s_base[256];
   __shared__ unsigned s_run[256];
-  // the scatter's per-warp digit counts, or a small batch's keys
-  __shared__ __align__(16) unsigned long long s_big[kSmallKeys];
-  int(*s_wc)[256] = reinterpret_cast<int(*)[256]>(s_big);
+  __shared__ int s_wc[kWarps][256];
+  extern __shared__ unsigned long long s_keys[];  // a small batch's keys
   __shared__ int s_sw[kWarps + 1];
   __shared__ long long s_swll[kWarps];
   __shared__ int s_flag;
-  __shared__ int s_small[2];
+  __shared__ int s_small[3];
 
   DevState* st = p.st;
   const GraphDev g = p.g;
@@ -229,10 +288,10 @@ __global__ void __launch_bounds__(kThreads) struct_kernel(StructParams p) {
     st->t_struct[0] = globaltimer_ns();
     pool0 = st->pool_used;
   }
-  const bool small = N <= kSmallKeys;
+  const bool front = N <= p.small_keys, small = front && N <= kTailKeys;
   long long NN = 0, NT_ = 0;
-  if (small) {
-    if (blockIdx.x == 0) small_front(p, s_big, (int)K, s_sw, s_small);
+  if (front) {
+    if (blockIdx.x == 0) small_front(p, s_keys, (int)K, s_wc, s_sw, s_small);
     if (!grid_sync(st, bar, p.bar_timeout_ns)) return;
     if (const unsigned bad = ld_cg(&st->status) & (ST_INVAL | ST_OVERFLOW)) {
       if (leader) st->pre_status = bad;
@@ -340,7 +399,7 @@ __global__ void __launch_bounds__(kThreads) struct_kernel(StructParams p) {
               rr[j] = 0;
               const unsigned act = __ballot_sync(0xffffffffu, valid);
               if (valid) {
-                const unsigned peers = __match_any_sync(act, dd[j]);
+                const unsigned peers = same_digit(act, (unsigned)dd[j]);
                 const int leader = __ffs(peers) - 1;
                 const int before = s_wc[w][dd[j]];
                 rr[j] = before + __popc(peers & lanemask_lt());
@@ -714,12 +773,15 @@ cudaError_t launch_struct(const StructParams& p, int grid, cudaStream_t s) {
   StructParams q = p;
   void* args[] = {&q};
   return cudaLaunchCooperativeKernel((const void*)struct_kernel, dim3(grid), dim3(kThreads), args,
-                                     0, s);
+                                     (size_t)p.small_keys * 2 * sizeof(unsigned long long), s);
 }
 
 int struct_kernel_occupancy() {
   int b = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, struct_kernel, kThreads, 0) != cudaSuccess)
+  if (cudaFuncSetAttribute(struct_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           kSmallKeys * 2 * (int)sizeof(unsigned long long)) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, struct_kernel, kThreads,
+                                                    kSmallKeys * 2 * sizeof(unsigned long long)) != cudaSuccess)
     return 0;
   return b;
 }

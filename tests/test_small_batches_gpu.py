@@ -1,6 +1,7 @@
 """Small batches are sorted, netted and cut into row units by one CTA in shared
-memory (up to 2048 lines); few relocation copies stay with that CTA, more go
-back to all of them; batches up to 32768 lines run on one CTA per SM.  At each
+memory (up to 2048 lines), which up to 512 lines also ends the batch; few
+relocation copies stay with that CTA then, more go back to all of them;
+batches up to 32768 lines run on one CTA per SM.  At each
 of these edges the adjacency, the degree property, the colours and the
 statistics must be the oracle's.
 
@@ -35,7 +36,7 @@ def _lines(rng, n, k, a, b, p_del):
 
 
 @pytest.mark.parametrize("variant,ov", [(dc.HI, po.HI), (dc.HB, po.HB)])
-@pytest.mark.parametrize("k", [0, 1, 2, 31, 1023, 1024, 1025, 2047, 2048, 2049, 32768, 32769])
+@pytest.mark.parametrize("k", [0, 1, 2, 31, 511, 512, 513, 1024, 2047, 2048, 2049, 32768, 32769])
 @pytest.mark.parametrize("kw", [{}, dict(cuda_graph=True), dict(grid_ctas=1)])
 def test_batches_at_the_edges_of_the_small_path(variant, ov, k, kw):
     n, a, b = er_graph(5000, 12, seed=4)
