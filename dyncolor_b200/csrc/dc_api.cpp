@@ -402,6 +402,17 @@ constexpr long long kOneCtaPerSmLines = 32768;
 int struct_grid(const dc_ctx* ctx, long long k) {
   return k <= kOneCtaPerSmLines ? std::min(ctx->grid_struct, ctx->sms) : ctx->grid_struct;
 }
+// CTAs of the recolour launch.  HI's phases on a small graph do not fill half
+// of the GPU's warps, and their barriers cost less with half the CTAs: R-MAT
+// scale 16 (65,536 vertices), 20k lines, 2.9 -> 2.7 ms, 20 lines on 1000
+// vertices 0.287 -> 0.275; scale 20 is 1 % and scale 24 17 % slower with one
+// CTA per SM.  HB's frontiers cover most of any graph (scale 16: 10 % slower).
+constexpr int kOneCtaVertices = 65536;
+int recolor_grid(const dc_ctx* ctx) {
+  return ctx->opt.variant == DC_HI && ctx->n <= kOneCtaVertices ? std::min(ctx->grid_recolor, ctx->sms)
+                                                                : ctx->grid_recolor;
+}
+
 // Enqueues one attempt of a batch (or load) on the context's stream, ending
 // with the copy of the device state into pinned host memory.  k_dev, when
 // set, makes the kernels read the line count from device memory, so a
@@ -438,7 +449,7 @@ dc_status enqueue_batch(dc_ctx* ctx, const dc_change* d_ch, const int* la, const
     }
     else
       rp.hri.min_live = 0;  // this batch scans every row
-    DC_CK(launch_recolor(rp, ctx->grid_recolor, ctx->stream));
+    DC_CK(launch_recolor(rp, recolor_grid(ctx), ctx->stream));
   }
   if (events) DC_CK(cudaEventRecord(ctx->ev1, ctx->stream));
   DC_CK(cudaMemcpyAsync(ctx->h_st, ctx->st, sizeof(DevState), cudaMemcpyDeviceToHost, ctx->stream));
@@ -489,7 +500,9 @@ dc_status run_batch(dc_ctx* ctx, const dc_change* d_ch, const int* la, const int
   // launch; it pays off when the batch is large enough to start long
   // cascades through those rows, and a small batch on a big graph (or one
   // graph's batch in a pool of many) would mostly pay for the build.
-  ctx->use_index = recolor && ctx->hri.min_live > 0 &&
+  // A row has fewer than n live slots: a graph of up to min_live vertices has
+  // nothing to index (the build's five launches took 11 us of a 280 us batch).
+  ctx->use_index = recolor && ctx->hri.min_live > 0 && ctx->n > ctx->hri.min_live &&
                    k * kIndexBatchRatio >= (ctx->index_n > 0 ? ctx->index_n : (long long)ctx->n);
   bool compacted = false;
   for (int attempt = 0;; ++attempt) {

@@ -111,3 +111,27 @@ def test_an_invalid_line_leaves_the_graph_as_it_was(at):
     assert np.array_equal(ctx.colors(), g.colors()) and sg.iterations == so.iterations
     assert np.array_equal(ctx.prop(), g.prop())
     ctx.close()
+
+
+@pytest.mark.parametrize("variant,ov", [(dc.HI, po.HI), (dc.HB, po.HB)])
+@pytest.mark.parametrize("n", [64, 65, 66, 65536, 65537])
+def test_graphs_at_the_edges_of_the_launch_rules(variant, ov, n):
+    """No index where no row can be long enough (n <= heavy_min_live), and one
+    CTA per SM for HI up to 65536 vertices."""
+    hub = np.arange(1, min(n, 3000), dtype=np.int32)
+    a, b = dc.uniform_pairs(n, 4 * n, seed=6)
+    a, b = dc.dedup(n, np.concatenate([a, np.zeros_like(hub)]), np.concatenate([b, hub]))
+    col = dc.greedy_color(n, a, b)
+    ctx = dc.Context(variant=variant, heavy_min_live=64)
+    ctx.load_edges(n, a, b)
+    ctx.set_colors(col)
+    g = oracle_graph(n, a, b, col)
+    rng = np.random.default_rng(n)
+    for _ in range(3):
+        ch = _lines(rng, n, max(30, n // 8), a, b, 0.5)
+        rc, so = g.apply_batch(ch, ov, po.SNAPSHOT)
+        sg = ctx.apply_batch(to_dc_changes(ch))
+        assert rc == po.OK and np.array_equal(ctx.colors(), g.colors())
+        assert (sg.iterations, sg.seed_targets, sg.frontier_total) == (
+            so.iterations, so.seed_targets, so.frontier_total)
+    ctx.close()
