@@ -440,11 +440,9 @@ dc_status enqueue_batch(dc_ctx* ctx, const dc_change* d_ch, const int* la, const
     }
     RecolorParams rp = recolor_params(ctx, d_ch, k);
     rp.k_dev = k_dev;
-    rp.ranges = ctx->index_n > 0 ? ctx->d_ranges : nullptr;
     if (ctx->use_index) {
       HriBufs hb = ctx->hri;
       hb.ranges = ctx->index_n > 0 ? ctx->d_ranges : nullptr;
-      rp.hri.ranges = hb.ranges;
       DC_CK(launch_hri_build(graph_dev(ctx), hb, ctx->st, ctx->opt.variant, ctx->stream));
     }
     else

@@ -237,7 +237,6 @@ struct RecolorParams {
   HriBufs hri;             // HI: heavy-row index (hri.min_live == 0: off)
   unsigned char* lflag;  // k
   int* pred;             // initial colouring: neighbours still to be coloured before each vertex
-  const int* ranges;     // vertex ranges of the launch's graphs (HriBufs::ranges layout), nullptr: all
   // Batched mode: the graph is a disjoint union of independent graphs.
   const int* gid;        // vertex -> graph (nullptr: one graph)
   int ngraphs;

@@ -46,11 +46,12 @@
 //   16 M adjacency entries where walking the frontier's rows (indexed ones by
 //   their candidates) visits 50 M, HB 0.1 G where that visits 0.5 G.  Measured
 //   with all of it, ms of device time per batch, before -> after: R-MAT scale
-//   24, 1 M lines, HI 157 -> 89; scale 22, 250 k lines, HB 331 -> 82; Chung-Lu
-//   1 M vertices, 250 k lines, HB 66 -> 17, HI 17 -> 16; R-MAT scale 16, 20 k
-//   lines, HI 4.8 -> 3.6, HB 6.6 -> 3.1.  What bounds the loop then is the
+//   24, 1 M lines, HI 157 -> 75; scale 22, 250 k lines, HB 331 -> 69; Chung-Lu
+//   1 M vertices, 250 k lines, HB 66 -> 15, HI 17 -> 14; R-MAT scale 16, 20 k
+//   lines, HI 4.8 -> 2.9, HB 6.6 -> 3.0.  What bounds the loop then is the
 //   chain of dependent L2 round trips in each of its three phases and their
-//   barriers: 7 us a phase when a few rows are left.
+//   barriers, 3.5 us for a phase with nothing to do and 6 to 10 for one with a
+//   few rows; and for HB on large graphs the dirty walks (see push_dirty).
 //
 // Heavy-row index (built by dc_hri.cu before the launch, for batches large
 // enough to use it): HI reads an indexed row through its colour-ordered copy
@@ -149,7 +150,6 @@ struct Shared {
   int cbuf[kCtaBuf];                  // the CTA's vertices to push, moved on at the end of the phase
   int mbuf[kMemBuf];                  // the CTA's new members
   unsigned ccnt, mcnt;                // entries claimed in cbuf and mbuf (may pass their sizes)
-  int sw[kWarps + 1];                 // block-scan scratch
   unsigned qn[2], qbase[4];           // the CTA's bulk push: items and units, queue, row-list and member positions
   int ok;                             // the last grid barrier did not time out
   unsigned bar;                       // arrivals the last grid barrier waited for
