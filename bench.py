@@ -346,7 +346,8 @@ def roofline_of(stats, K, hi: bool, k_lines: int, traffic_per_entry=None) -> dic
            "entries_covered_per_launch": scanned / K,
            "entries_read_per_launch": sum(s.slots_read for s in stats) / K,
            "note": f"{per_slot} B per covered adjacency entry (id + neighbour colour"
-                   + ("" if hi else " + priority") + "), covered entries counted on the device"}
+                   + ("" if hi else " + priority") + "), covered entries counted on the device; the loop visits only "
+                   "rows where something can have changed, so this is the rules' work per second and may pass the peak"}
     if traffic is not None:
         # measured DRAM bytes of a launch over its duration, against the peak
         out["dram_gbs"] = traffic / (dom_ms / K / 1e3) / 1e9
