@@ -1430,7 +1430,7 @@ __device__ __noinline__ int find_witness(bool need, int u, int cu, unsigned at, 
   __syncwarp();
   T.excl[lane_id()] = sp.len;
   __syncwarp();
-  unsigned todo = __ballot_sync(0xffffffffu, need && !shrt);
+  unsigned todo = __ballot_sync(0xffffffffu, need && !shrt && inl > 0);
 #pragma unroll 1
   while (todo) {
     const int l = __ffs(todo) - 1;
